@@ -63,13 +63,11 @@ struct DBuf {
   }
 };
 
-// Source chunks per target leaf of the FP64 near field: 1 at large n; at small n (few target
-// leaves, ~48 bodies each) enough chunks for ~32 warps per SM, at most 16.  A function of n only,
-// so the direct launches and a captured graph of the same call sum in the same order.
-static inline int p2p_nsplit(int n) {
-  long long k = (148LL * 32 * 48 + n - 1) / (n > 0 ? n : 1);
-  return (int)(k < 1 ? 1 : k > 16 ? 16 : k);
-}
+// Near-field work units K (tc_p2p.cuh): rows of more than 1 / K of the whole cost are split.  About
+// six items per resident warp (148 SMs x 20 warps) keep the launch's end short; below 8,192 bodies
+// items that small would hold less than two tiles of sources.  A function of n only, so the direct
+// launches and a captured graph agree.
+static inline int p2p_units(int n) { return 148 * (n < 8192 ? 32 : 128); }
 
 // what a captured evaluation was recorded for (a call must match to replay it)
 struct TcGraphKey {
@@ -155,7 +153,12 @@ struct tc_ctx {
   // tc_direct_sums: bodies in caller order, targets, partial and final sums
   DBuf<double> ds_bod, ds_out;
   DBuf<double> diag;  // system diagnostics: block partials + the 9 results
-  DBuf<double> p2p_part;  // near-field partial sums per source chunk (few target leaves)
+  // near-field work items (tc_p2p.cuh): source bodies per target, unsplit rows, chunks of split rows
+  DBuf<int> p2p_s;
+  DBuf<int2> p2p_singles;
+  DBuf<TcP2PItem> p2p_items;
+  DBuf<TcP2PRow> p2p_rows;
+  DBuf<double> p2p_slots;  // their sums; below kP2PSmallN bodies the chunk sums
   // block-time-step integrator: accelerations, potential, 1/tau^4 sums; split counters, pair
   // positions, kick flags
   DBuf<double> ev_d;
@@ -175,7 +178,8 @@ struct tc_ctx {
   TcTravCounters* d_cnt = nullptr;
   unsigned int* d_err = nullptr;
   unsigned int* d_small = nullptr;  // [0] m2l targets, [1] p2p targets, [2] leaves, [9] tensor M2L counter,
-                                    // [10] target counter of the persistent FP64 M2L (graph)
+                                    // [10] target counter of the persistent FP64 M2L (graph), [4..6] near-field
+                                    // items, unsplit rows, split rows, [12] near-field work counter
   DBuf<float> tc_bins;  // tensor-core M2L bin matrices (hi, lo) of order tc_bins_q
   int tc_bins_q = -1;
   long long wait_limit = kTcWaitLimit;  // clock cycles a bounded device wait may take (tc_set_wait_limit)
@@ -396,11 +400,6 @@ __global__ void k_identity(int n, int* v) {
   if (i < n) v[i] = i;
 }
 
-__global__ void k_nan_check(int n, const double* x, const double* y, const double* z, const double* m, unsigned* err) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && !(isfinite(x[i]) && isfinite(y[i]) && isfinite(z[i]) && isfinite(m[i]))) tc_set_err(err, TC_EBIT_NAN);
-}
-
 __global__ void k_leaf_list(int ncell, const int* nchild, int* leaves, unsigned* cnt, const int* ncdev = nullptr) {
   if (ncdev) ncell = *ncdev;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -413,19 +412,79 @@ __global__ void k_leaf_list(int ncell, const int* nchild, int* leaves, unsigned*
   if (has) leaves[base + __popc(mask & ((1u << lane) - 1u))] = i;
 }
 
-// sum over the P2P list of (sink-cell bodies) x (source-cell bodies)
-__global__ void k_p2p_count(const unsigned long long* __restrict__ keys, unsigned long long n, int sbits,
-                            const int* __restrict__ nbody, const uint8_t* __restrict__ has_sink,
-                            unsigned long long* total, const unsigned long long* ndev = nullptr) {
-  if (ndev && *ndev < n) n = *ndev;
-  unsigned long long loc = 0, mask = (1ull << sbits) - 1ull;
-  for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (unsigned long long)gridDim.x * blockDim.x) {
-    int t = (int)(keys[k] >> sbits), s = (int)(keys[k] & mask);
-    if (has_sink[t]) loc += (unsigned long long)nbody[t] * (unsigned long long)nbody[s];
+// whether a body can be in several target cells of the near field (tc_p2p_add)
+static bool p2p_shared(const tc_ctx* ctx) { return ctx->prm.variant == TC_VARIANT_TOP && ctx->prm.ncrit < 8; }
+
+// whether the near field runs in the fixed chunks of small systems (k_p2p_chunks); the time-step pass
+// never does
+static bool p2p_chunked(const tc_ctx* ctx, int n) {
+  return n < kP2PSmallN && ctx->prm.precision == TC_PREC_FP64 && !p2p_shared(ctx);
+}
+
+// buffers of the near field's work items: nc cells (targets), NC sums per body
+static cudaError_t p2p_reserve(tc_ctx* ctx, int n, size_t nc, int NC) {
+  if (p2p_chunked(ctx, n) && NC != 5) return ctx->p2p_slots.ensure((size_t)kP2PChunks * NC * n);
+  const size_t cap = 2 * (size_t)p2p_units(n);
+  cudaError_t e = ctx->p2p_s.ensure(nc);
+  if (e == cudaSuccess) e = ctx->p2p_singles.ensure(nc + (size_t)n / 32 + 1);
+  if (e == cudaSuccess) e = ctx->p2p_items.ensure(cap);
+  if (e == cudaSuccess) e = ctx->p2p_rows.ensure(cap);
+  if (e == cudaSuccess) e = ctx->p2p_slots.ensure(cap * NC * 32);
+  return e;
+}
+
+// the work items of the near field over the target list (p2p_reserve done); frontier[0] of the
+// traversal counters receives the pair count
+static TcP2PWork p2p_plan(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* ntldev) {
+  cudaStream_t st = ctx->stream;
+  unsigned* cnt = ctx->d_small + 4;
+  cudaMemsetAsync(ctx->d_cnt, 0, 2 * sizeof(unsigned long long), st);  // frontier[0], frontier[1]
+  cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), st);
+  cudaMemsetAsync(ctx->d_small + 12, 0, sizeof(unsigned), st);
+  unsigned long long *inter = &ctx->d_cnt->frontier[0], *cost = &ctx->d_cnt->frontier[1];
+  const int gw = std::min(nblocks(ntl, 8), 148 * 8), gp = gw;
+  k_p2p_work<<<gw, 256, 0, st>>>(ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, cv, ctx->p2p_s.p, inter, cost,
+                                 ntldev);
+  const int K = p2p_units(n);
+  k_p2p_plan<<<gp, 256, 0, st>>>(ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, cv, ctx->p2p_s.p, cost, K,
+                                 2 * K, ctx->p2p_singles.p, ctx->p2p_items.p, ctx->p2p_rows.p, cnt, ntldev);
+  TcP2PWork W;
+  W.items = ctx->p2p_items.p;
+  W.singles = ctx->p2p_singles.p;
+  W.cnt = cnt;
+  W.next = ctx->d_small + 12;
+  W.slots = ctx->p2p_slots.p;
+  W.shared = p2p_shared(ctx);
+  return W;
+}
+
+// the near field itself: a persistent grid over the items, then the split rows folded
+template <bool JERK>
+static void p2p_run(tc_ctx* ctx, TcBodies b, TcCells cv, TcOut o, int n, int ntl, const unsigned* ntldev) {
+  cudaStream_t st = ctx->stream;
+  if (p2p_chunked(ctx, n)) {
+    // the pair count, then the fixed chunks
+    cudaMemsetAsync(ctx->d_cnt, 0, 2 * sizeof(unsigned long long), st);
+    k_p2p_chunks<JERK><<<nblocks((long long)ntl * kP2PChunks, kP2PWarps), kP2PWarps * 32, 0, st>>>(
+        ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o, ntldev, kP2PChunks, ctx->p2p_slots.p, n,
+        &ctx->d_cnt->frontier[0]);
+    k_p2p_chunks_join<JERK><<<nblocks(ntl, kP2PWarps), kP2PWarps * 32, 0, st>>>(
+        ctx->p2p_tl.p, ntl, b, cv, o, kP2PChunks, ctx->p2p_slots.p, n, ntldev);
+    ctx->launches += 2;
+    return;
   }
-  for (int o = 16; o > 0; o >>= 1) loc += __shfl_xor_sync(0xffffffffu, loc, o);
-  if ((threadIdx.x & 31) == 0 && loc) atomicAdd(total, loc);
+  const TcP2PWork W = p2p_plan(ctx, cv, n, ntl, ntldev);
+  if (ctx->prm.precision != TC_PREC_FP64) {
+    k_body_f32<JERK><<<nblocks(n, 256), 256, 0, st>>>(n, b);
+    k_p2p_mixed<JERK><<<148 * 7, kP2PWarps * 32, 0, st>>>(ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o, kP2PExclFrac,
+                                                          W);
+    ctx->launches++;
+  } else {
+    k_p2p<JERK><<<148 * (JERK ? 4 : 5), kP2PWarps * 32, 0, st>>>(ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o, W);
+  }
+  k_p2p_join<JERK ? 7 : 4, false><<<148 * 4, kP2PWarps * 32, 0, st>>>(ctx->p2p_rows.p, W.cnt, b, cv, o, nullptr,
+                                                                       W.slots, W.shared);
+  ctx->launches += 4;
 }
 
 // ----------------------------------------------------------------------------------------
@@ -820,15 +879,11 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
     k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->m2l.p, nm, ctx->ncell, sbits, ctx->m2l_start.p, ctx->m2l_src.p);
     k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->p2p.p, np, ctx->ncell, sbits, ctx->p2p_start.p, ctx->p2p_src.p);
     TC_CK(cudaMemsetAsync(ctx->d_small, 0, 4 * sizeof(unsigned), st));
-    TC_CK(cudaMemsetAsync(&ctx->d_cnt->frontier[0], 0, sizeof(unsigned long long), st));
-    k_p2p_count<<<148 * 4, 256, 0, st>>>(ctx->p2p.p, np, sbits, cv.nbody, cv.has_sink, &ctx->d_cnt->frontier[0]);
-    ctx->launches++;
     k_list_targets<<<nblocks(ctx->ncell, 256), 256, 0, st>>>(ctx->m2l_start.p, ctx->ncell, ctx->m2l_tl.p, ctx->d_small);
     k_list_targets<<<nblocks(ctx->ncell, 256), 256, 0, st>>>(ctx->p2p_start.p, ctx->ncell, ctx->p2p_tl.p, ctx->d_small + 1);
     k_leaf_list<<<nblocks(ctx->ncell, 256), 256, 0, st>>>(ctx->ncell, cv.nchild, ctx->leaves.p, ctx->d_small + 2);
   }
   TC_CK(cudaMemcpyAsync(hs, ctx->d_small, sizeof(hs), cudaMemcpyDeviceToHost, st));
-  TC_CK(cudaMemcpyAsync(&ctx->n_inter, &ctx->d_cnt->frontier[0], sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   TC_CK(cudaStreamSynchronize(st));
     return TC_OK;
   };
@@ -896,7 +951,6 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
   TcOut o = out_view(ctx, n, JERK);
   TC_CK(cudaMemsetAsync(ctx->outs.p, 0, sizeof(double) * (size_t)n * (JERK ? 7 : 4), st));
   const bool mixed = prm.precision == TC_PREC_MIXED_M2L;              // FP32 far field
-  const bool mixed_p2p = prm.precision != TC_PREC_FP64;               // FP32 near field
   ctx->n_classes = 1;
   ctx->class_order[0] = P;
   ctx->class_pairs[0] = (long long)ctx->n_m2l;
@@ -962,49 +1016,25 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
     TC_CK(ctx->tsum.ensure((size_t)n));
     TC_CK(cudaMemsetAsync(ctx->tsum.p, 0, sizeof(double) * (size_t)n, st));
   }
-  if (hs[1] > 0 && ctx->steps) {
-    if constexpr (!JERK) {
-      const int ntl = (int)hs[1];
-      int nsplit = p2p_nsplit(n);  // few target leaves: source chunks folded in order, as k_p2p
-      if (nsplit > 1 && ctx->p2p_part.ensure((size_t)nsplit * 5 * n) != cudaSuccess) nsplit = 1;
-      if (nsplit > 1) {
-        k_p2p_steps<<<nblocks(ntl * nsplit, kP2PWarps), kP2PWarps * 32, 0, st>>>(
-            ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o, ctx->dt_param, ctx->tsum.p, nsplit,
-            ctx->p2p_part.p, n);
-        k_p2p_steps_join<<<nblocks(ntl, kP2PWarps), kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, ntl, b, cv, o,
-                                                                             ctx->tsum.p, nsplit, ctx->p2p_part.p, n);
-        ctx->launches++;
-      } else {
-        k_p2p_steps<<<nblocks(ntl, kP2PWarps), kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, ntl, ctx->p2p_start.p,
-                                                                        ctx->p2p_src.p, b, cv, o, ctx->dt_param,
-                                                                        ctx->tsum.p);
-      }
-      ctx->launches++;
+  ctx->n_inter = 0;
+  if (hs[1] > 0) {
+    TC_CK(p2p_reserve(ctx, n, (size_t)ctx->ncell, ctx->steps ? 5 : JERK ? 7 : 4));
+    if (!ctx->steps) {
+      p2p_run<JERK>(ctx, b, cv, o, n, (int)hs[1], nullptr);
+    } else if constexpr (!JERK) {
+      const TcP2PWork W = p2p_plan(ctx, cv, n, (int)hs[1], nullptr);
+      if (ctx->dt_param > 0.0 && std::isfinite(1.0 / ctx->dt_param) && std::isfinite(ctx->dt_param))
+        k_p2p_steps<true><<<148 * 5, kP2PWarps * 32, 0, st>>>(ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o,
+                                                              ctx->dt_param, ctx->tsum.p, W);
+      else
+        k_p2p_steps<false><<<148 * 5, kP2PWarps * 32, 0, st>>>(ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o,
+                                                               ctx->dt_param, ctx->tsum.p, W);
+      k_p2p_join<5, true><<<148 * 4, kP2PWarps * 32, 0, st>>>(ctx->p2p_rows.p, W.cnt, b, cv, o, ctx->tsum.p, W.slots,
+                                                               W.shared);
+      ctx->launches += 4;
     }
-  } else if (hs[1] > 0) {
-    int g = nblocks(hs[1], kP2PWarps);
-    if (mixed_p2p) {
-      k_body_f32<JERK><<<nblocks(n, 256), 256, 0, st>>>(n, b);
-      ctx->launches++;
-      k_p2p_mixed<JERK><<<g, kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, (int)hs[1], ctx->p2p_start.p, ctx->p2p_src.p, b,
-                                                       cv, o, kP2PExclFrac);
-    } else {
-      // few target leaves (small n): split each leaf's sources over up to 16 warps, then fold
-      // the chunks in order (k_p2p_join); the split depends on n only, as in the graph path
-      const int ntl = (int)hs[1];
-      int nsplit = p2p_nsplit(n);
-      constexpr int NC = JERK ? 7 : 4;
-      if (nsplit > 1 && ctx->p2p_part.ensure((size_t)nsplit * NC * n) != cudaSuccess) nsplit = 1;
-      if (nsplit > 1) {
-        k_p2p<JERK><<<nblocks(ntl * nsplit, kP2PWarps), kP2PWarps * 32, 0, st>>>(
-            ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o, nullptr, nsplit, ctx->p2p_part.p, n);
-        k_p2p_join<JERK><<<g, kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, ntl, b, cv, o, nsplit, ctx->p2p_part.p, n);
-        ctx->launches++;
-      } else {
-        k_p2p<JERK><<<g, kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o);
-      }
-    }
-    ctx->launches++;
+    TC_CK(cudaMemcpyAsync(&ctx->n_inter, &ctx->d_cnt->frontier[0], sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                          st));
   }
   if (ctx->events) cudaEventRecord(ctx->ev[6], st);
   return TC_OK;
@@ -1094,14 +1124,11 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
   k_list_csr<<<148 * 8, 256, 0, st>>>(kp, ctx->pcap, ccap, sbits, ctx->p2p_start.p, ctx->p2p_src.p,
                                       &ctx->d_cnt->n_p2p, d_ncell);
   cudaMemsetAsync(ctx->d_small, 0, 4 * sizeof(unsigned), st);
-  cudaMemsetAsync(&ctx->d_cnt->frontier[0], 0, sizeof(unsigned long long), st);
-  k_p2p_count<<<148 * 4, 256, 0, st>>>(kp, ctx->pcap, sbits, cv.nbody, cv.has_sink, &ctx->d_cnt->frontier[0],
-                                       &ctx->d_cnt->n_p2p);
   k_list_targets<<<nblocks(ccap, 256), 256, 0, st>>>(ctx->m2l_start.p, ccap, ctx->m2l_tl.p, ctx->d_small, d_ncell);
   k_list_targets<<<nblocks(ccap, 256), 256, 0, st>>>(ctx->p2p_start.p, ccap, ctx->p2p_tl.p, ctx->d_small + 1,
                                                      d_ncell);
   k_leaf_list<<<nblocks(ccap, 256), 256, 0, st>>>(ccap, cv.nchild, ctx->leaves.p, ctx->d_small + 2, d_ncell);
-  L += 6;
+  L += 5;
   graph_check(ctx, "list sort and offsets");
   graph_event(ctx, 3, st);
   // ---- far field and near field
@@ -1132,31 +1159,9 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
   L += TC_MAX_LEVEL + 1;
   graph_check(ctx, "downward pass");
   graph_event(ctx, 5, st);
-  {
-    const int g = nblocks(ccap, kP2PWarps);  // a warp per target slot; warps past the count exit
-    if (prm.precision != TC_PREC_FP64) {
-      k_body_f32<JERK><<<nblocks(n, 256), 256, 0, st>>>(n, b);
-      L++;
-    }
-    if (prm.precision != TC_PREC_FP64)
-      k_p2p_mixed<JERK><<<g, kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, ccap, ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o,
-                                                       kP2PExclFrac, ctx->d_small + 1);
-    else {
-      const int nsplit = p2p_nsplit(n);
-      if (nsplit > 1) {  // the same chunks as the direct launches (p2p_part sized by graph_plan)
-        k_p2p<JERK><<<nblocks(ccap * nsplit, kP2PWarps), kP2PWarps * 32, 0, st>>>(
-            ctx->p2p_tl.p, ccap, ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o, ctx->d_small + 1, nsplit,
-            ctx->p2p_part.p, n);
-        k_p2p_join<JERK><<<g, kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, ccap, b, cv, o, nsplit, ctx->p2p_part.p, n,
-                                                        ctx->d_small + 1);
-        L++;
-      } else {
-        k_p2p<JERK><<<g, kP2PWarps * 32, 0, st>>>(ctx->p2p_tl.p, ccap, ctx->p2p_start.p, ctx->p2p_src.p, b, cv, o,
-                                                   ctx->d_small + 1);
-      }
-    }
-  }
-  L += 2;
+  const long long before = ctx->launches;
+  p2p_run<JERK>(ctx, b, cv, o, n, ccap, ctx->d_small + 1);  // buffers reserved by graph_plan
+  L += ctx->launches - before;
   graph_check(ctx, "P2P");
   graph_event(ctx, 6, st);
   ctx->glaunches += L;
@@ -1355,33 +1360,64 @@ struct TcNoallocDev {
 static TcNoallocDev g_noalloc_dev[64];
 static std::mutex g_noalloc_mu;  // guards the one-time fill of g_noalloc_dev
 
-// Direct-sum evaluation over working storage the caller provides: S entries per array in
-// `scratch` (14 arrays: x y z m vx vy vz | pot ax ay az jx jy jz), `index` and `flags`
-// (n <= S).  Shared by tc_evaluate_direct_noalloc (the static array) and the block-time-step
-// integrator's direct kicks (the context's own buffers, so contexts never share storage).
+// whether any of the n-entry outputs shares memory with an input (the direct kernel reads the
+// inputs while it writes the outputs)
+static bool outputs_overlap(int n, const double* const* in, int nin, const unsigned char* flags, double* const* out,
+                            int nout) {
+  const uintptr_t len = (uintptr_t)n * sizeof(double);
+  for (int o = 0; o < nout; o++) {
+    const uintptr_t a = (uintptr_t)out[o];
+    if (!a) continue;
+    for (int i = 0; i < nin; i++) {
+      const uintptr_t c = (uintptr_t)in[i];
+      if (c && a < c + len && c < a + len) return true;
+    }
+    const uintptr_t f = (uintptr_t)flags;
+    if (f && a < f + (uintptr_t)n && f < a + len) return true;
+  }
+  return false;
+}
+
+static void direct_launch(int n, const double* x, const double* y, const double* z, const double* vx,
+                          const double* vy, const double* vz, const double* m, const unsigned char* flags,
+                          double eps2, TcOut o, bool jerk, unsigned* err, cudaStream_t st) {
+  if (jerk)
+    k_direct<true><<<nblocks(n, kDirT), kDirThreads, 0, st>>>(n, x, y, z, vx, vy, vz, m, flags, eps2, o, err);
+  else
+    k_direct<false><<<nblocks(n, kDirT), kDirThreads, 0, st>>>(n, x, y, z, vx, vy, vz, m, flags, eps2, o, err);
+}
+
+// Direct-sum evaluation that allocates nothing.  Where an output shares memory with an input, the
+// inputs are first copied to working storage the caller provides: S entries per array in
+// `scratch` (7 arrays: x y z m vx vy vz), `index` and `flags` (n <= S).  Shared by
+// tc_evaluate_direct_noalloc (the static array) and the block-time-step integrator's direct kicks.
 static cudaError_t direct_with_scratch(int n, const double* x, const double* y, const double* z, const double* vx,
                                        const double* vy, const double* vz, const double* m,
                                        const unsigned char* flags, double* ax, double* ay, double* az, double* pot,
                                        double* jx, double* jy, double* jz, int jerk, cudaStream_t st,
                                        double* scratch, int* index, uint8_t* fl, size_t S, double eps2 = 0.0) {
+  TcOut o;
+  o.pot = pot; o.ax = ax; o.ay = ay; o.az = az;
+  o.jx = jerk ? jx : nullptr; o.jy = jerk ? jy : nullptr; o.jz = jerk ? jz : nullptr;
+  const double* in[7] = {x, y, z, m, vx, vy, vz};
+  double* outs[7] = {ax, ay, az, pot, o.jx, o.jy, o.jz};
+  if (!outputs_overlap(n, in, jerk ? 7 : 4, flags, outs, 7)) {
+    if (!jerk && n <= kChainN) {
+      k_direct_chain<<<nblocks(n, kChainT), 256, 0, st>>>(n, x, y, z, m, flags, eps2, o);
+      return cudaGetLastError();
+    }
+    direct_launch(n, x, y, z, vx, vy, vz, m, flags, eps2, o, jerk != 0, nullptr, st);
+    return cudaGetLastError();
+  }
   TcBodies b;
   b.x = scratch; b.y = scratch + S; b.z = scratch + 2 * S; b.m = scratch + 3 * S;
   b.vx = jerk ? scratch + 4 * S : nullptr; b.vy = jerk ? scratch + 5 * S : nullptr;
   b.vz = jerk ? scratch + 6 * S : nullptr;
   b.flags = fl;
   b.perm = index;
-  b.eps2 = eps2;
-  TcOut o;
-  o.pot = scratch + 7 * S; o.ax = scratch + 8 * S; o.ay = scratch + 9 * S; o.az = scratch + 10 * S;
-  o.jx = jerk ? scratch + 11 * S : nullptr; o.jy = jerk ? scratch + 12 * S : nullptr;
-  o.jz = jerk ? scratch + 13 * S : nullptr;
   k_identity<<<nblocks(n, 256), 256, 0, st>>>(n, index);
   k_gather_bodies<<<nblocks(n, 256), 256, 0, st>>>(n, index, x, y, z, m, vx, vy, vz, flags, b);
-  if (jerk)
-    k_direct<true><<<nblocks(n, 128), 128, 0, st>>>(n, b, o);
-  else
-    k_direct<false><<<nblocks(n, 128), 128, 0, st>>>(n, b, o);
-  k_scatter_out<<<nblocks(n, 256), 256, 0, st>>>(n, index, o, pot, ax, ay, az, jerk ? jx : nullptr, jy, jz);
+  direct_launch(n, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.m, b.flags, eps2, o, jerk != 0, nullptr, st);
   return cudaGetLastError();
 }
 
@@ -1490,7 +1526,8 @@ tc_status tc_destroy(tc_ctx* ctx) {
   ctx->cell_pn.release(); ctx->cls_start.release(); ctx->cls_tl.release(); ctx->mlp_w.release();
   ctx->judge_idx.release(); ctx->judge_out.release();
   ctx->ds_bod.release(); ctx->ds_out.release(); ctx->ds_flags.release(); ctx->ds_idx.release(); ctx->ds_tgt.release();
-  ctx->tsum.release(); ctx->diag.release(); ctx->p2p_part.release();
+  ctx->tsum.release(); ctx->diag.release(); ctx->p2p_s.release(); ctx->p2p_singles.release();
+  ctx->p2p_items.release(); ctx->p2p_rows.release(); ctx->p2p_slots.release();
   ctx->ev_d.release(); ctx->ev_u.release(); ctx->ev_i.release(); ctx->ev_f.release();
   ctx->amag.release(); ctx->body_scale.release(); ctx->cell_scale.release(); ctx->m2l_src2.release();
   ctx->m2l_off.release(); ctx->cls_rng.release(); ctx->cell_feat.release(); ctx->kd_scratch.release(); ctx->kd_index.release(); ctx->kd_flags.release();
@@ -1641,15 +1678,37 @@ static tc_status evaluate_impl(tc_ctx* ctx, int n, const double* x, const double
   TcBodies b = bodies_view(ctx, n, jerk);
   TcOut o = out_view(ctx, n, jerk);
   tc_status rs = TC_OK;
+  bool direct_out = false;  // a direct sum that wrote the caller's outputs itself
   if (ctx->direct) {
-    k_nan_check<<<nblocks(n, 256), 256, 0, st>>>(n, dx, dy, dz, dm, ctx->d_err);
-    k_identity<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->vals.p);
-    k_gather_bodies<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->vals.p, dx, dy, dz, dm, dvx, dvy, dvz, df, b);
-    if (jerk)
-      k_direct<true><<<nblocks(n, 128), 128, 0, st>>>(n, b, o);
-    else
-      k_direct<false><<<nblocks(n, 128), 128, 0, st>>>(n, b, o);
-    ctx->launches += 4;
+    const double* in[7] = {dx, dy, dz, dm, dvx, dvy, dvz};
+    double* outp[7] = {ax, ay, az, pot, jx, jy, jz};
+    // the sums go straight from the caller's arrays to the caller's outputs, except where the judge
+    // needs both in the context or an output shares memory with an input
+    direct_out = ctx->prm.judge_n <= 0 && (mem == TC_MEM_HOST || !outputs_overlap(n, in, 7, df, outp, 7));
+    const double eps2 = ctx->prm.softening * ctx->prm.softening;
+    if (direct_out) {
+      TcOut u;
+      if (mem == TC_MEM_HOST) {  // the staged outputs, as below
+        TC_CK(ctx->out_d.ensure(8 * N));
+        double* s = ctx->out_d.p;
+        double* d[7] = {s + N, s + 2 * N, s + 3 * N, s, jx ? s + 4 * N : nullptr, jx ? s + 5 * N : nullptr,
+                        jx ? s + 6 * N : nullptr};
+        memcpy(outp, d, sizeof(d));
+      }
+      u.ax = outp[0]; u.ay = outp[1]; u.az = outp[2]; u.pot = outp[3];
+      u.jx = jerk && jx ? outp[4] : nullptr; u.jy = jerk && jx ? outp[5] : nullptr;
+      u.jz = jerk && jx ? outp[6] : nullptr;
+      direct_launch(n, dx, dy, dz, dvx, dvy, dvz, dm, df, eps2, u, jerk, ctx->d_err, st);
+      if (jx && !jerk) {  // jerk outputs of a tree without jerks are zero
+        for (double* p : {outp[4], outp[5], outp[6]}) TC_CK(cudaMemsetAsync(p, 0, N * sizeof(double), st));
+      }
+      ctx->launches++;
+    } else {
+      k_identity<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->vals.p);
+      k_gather_bodies<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->vals.p, dx, dy, dz, dm, dvx, dvy, dvz, df, b);
+      direct_launch(n, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.m, b.flags, eps2, o, jerk, ctx->d_err, st);
+      ctx->launches += 3;
+    }
     ctx->ncell = 0; ctx->nleaf = 0; ctx->n_m2l = 0; ctx->n_p2p = 0; ctx->max_level = 0;
     if (ctx->events)
       for (int i = 1; i <= 6; i++) cudaEventRecord(ctx->ev[i], st);
@@ -1720,8 +1779,10 @@ static tc_status evaluate_impl(tc_ctx* ctx, int n, const double* x, const double
     ojx = jx ? s + 4 * N : nullptr; ojy = jx ? s + 5 * N : nullptr; ojz = jx ? s + 6 * N : nullptr;
     ots = s + 7 * N;
   }
-  k_scatter_out<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->perm.p, o, opot, oax, oay, oaz, ojx, ojy, ojz);
-  ctx->launches++;
+  if (!direct_out) {
+    k_scatter_out<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->perm.p, o, opot, oax, oay, oaz, ojx, ojy, ojz);
+    ctx->launches++;
+  }
   const bool keep_amag = ctx->prm.selector > 0 && !timestep && !ctx->direct;
   if (keep_amag) {  // the next evaluation's per-target error budget
     TC_CK(ctx->amag.ensure(N));
@@ -1779,11 +1840,12 @@ static void graph_signature(const tc_ctx* c, std::vector<const void*>& s) {
                         c->split_off.p, c->expn.p,     c->front[0].p,  c->front[1].p,  c->m2l.p,
                         c->m2l_alt.p,  c->p2p.p,       c->p2p_alt.p,   c->m2l_start.p, c->m2l_src.p,
                         c->p2p_start.p, c->p2p_src.p,  c->m2l_tl.p,    c->p2p_tl.p,    c->leaves.p,
-                        c->judge_idx.p, c->judge_out.p, c->p2p_part.p, c->bpart.p,     c->tc_bins.p,
+                        c->judge_idx.p, c->judge_out.p, c->p2p_slots.p, c->bpart.p,    c->tc_bins.p,
+                        c->p2p_s.p,     c->p2p_singles.p, c->p2p_items.p, c->p2p_rows.p,
                         c->amag.p,      c->body_scale.p, c->cell_scale.p, c->m2l_src2.p, c->m2l_off.p,
                         c->cell_pn.p,   c->mlp_w.p,      c->cls_rng.p,    c->cell_feat.p};
   s.assign(bufs, bufs + sizeof(bufs) / sizeof(bufs[0]));
-  const size_t caps[] = {c->ccap, c->mcap, c->pcap, c->fcap, c->expn.n, c->p2p_part.n};
+  const size_t caps[] = {c->ccap, c->mcap, c->pcap, c->fcap, c->expn.n, c->p2p_slots.n};
   for (size_t v : caps) s.push_back((const void*)(uintptr_t)v);
 }
 
@@ -1926,7 +1988,7 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
       ctx->p2p_start.ensure(ccap + 1) || ctx->m2l_src.ensure(ctx->mcap + 1) || ctx->p2p_src.ensure(ctx->pcap + 1) ||
       ctx->m2l_tl.ensure(ccap) || ctx->p2p_tl.ensure(ccap) || ctx->leaves.ensure(ccap) ||
       ctx->expn.ensure(ccap * NT * (jerk ? 4 : 2)) || ctx->bpart.ensure(6 * 148 * 4) ||
-      (p2p_nsplit(n) > 1 && ctx->p2p_part.ensure((size_t)p2p_nsplit(n) * (jerk ? 7 : 4) * N)))
+      p2p_reserve(ctx, n, ccap, jerk ? 7 : 4))
     return;
   if (ctx->prm.selector > 0 &&
       (ctx->cell_pn.ensure(ccap * (ctx->prm.p + 1)) || ctx->cell_scale.ensure(ccap) || ctx->body_scale.ensure(N) ||
@@ -2528,7 +2590,11 @@ tc_status tc_get_cells(tc_ctx* ctx, int* begin, int* nbody, int* nchild, int* ch
     }
     if (R) TC_CK(cudaMemcpy(R, ctx->cdbl.p + 6 * cc, nc * sizeof(double), cudaMemcpyDeviceToHost));
   }
-  if (perm) TC_CK(cudaMemcpy(perm, ctx->perm.p, ctx->n * sizeof(int), cudaMemcpyDeviceToHost));
+  if (perm && ctx->direct) {
+    for (int i = 0; i < ctx->n; i++) perm[i] = i;
+  } else if (perm) {
+    TC_CK(cudaMemcpy(perm, ctx->perm.p, ctx->n * sizeof(int), cudaMemcpyDeviceToHost));
+  }
   return TC_OK;
 }
 
