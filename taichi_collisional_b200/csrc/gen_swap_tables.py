@@ -204,6 +204,22 @@ def write_header(mats, path):
             L.append("    o[%d] = %s;" % (k, " + ".join(terms) if terms else "T(0)"))
         L.append("  }")
         L.append("};")
+    L.append("// The same map between restricted orders: the rows |m| <= RO of the output from the inputs")
+    L.append("// |m| <= RI (the z-translation of an order-P M2L joins only m <= min(n, P - n)).")
+    L.append("#define TC_SW_I(j, c) if constexpr ((j > N ? j - N : N - j) <= RI) s += T(c) * v[j];")
+    L.append("#define TC_SW_O(k, ...) if constexpr ((k > N ? k - N : N - k) <= RO) { T s = T(0); __VA_ARGS__ o[k] = s; }")
+    L.append("template <int N> struct TcSwapPart;")
+    for n, S in enumerate(mats):
+        L.append("template <> struct TcSwapPart<%d> {" % n)
+        L.append("  static constexpr int N = %d;" % n)
+        L.append("  template <int RI, int RO, typename T> static __device__ __forceinline__ void apply(const T* v, T* o) {")
+        for k in range(2 * n + 1):
+            terms = ["TC_SW_I(%d, %s)" % (j, _fmt(S[k][j])) for j in range(2 * n + 1) if S[k][j] != 0]
+            L.append("    TC_SW_O(%d, %s)" % (k, " ".join(terms)))
+        L.append("  }")
+        L.append("};")
+    L.append("#undef TC_SW_I")
+    L.append("#undef TC_SW_O")
     L.append("// Orthogonal form used by the mixed-precision M2L: T_n = E S_n E^-1 with")
     L.append("// E = diag(sqrt((n+|m|)!(n-|m|)!) c_m / ((n+|m|)!(n-|m|)!)), c_0 = 1, c_m = sqrt(2).")
     L.append("template <int N> struct TcSwapOrthDeg;")

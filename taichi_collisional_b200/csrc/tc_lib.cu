@@ -26,6 +26,7 @@
 #include "tc_upward.cuh"
 #include "tc_traverse.cuh"
 #include "tc_m2l.cuh"
+#include "tc_m2l_warp.cuh"
 #include "tc_m2l_mixed.cuh"
 #include "tc_m2l_tc.cuh"
 #include "tc_emac.cuh"
@@ -115,6 +116,7 @@ struct tc_ctx {
   DBuf<uint8_t> csink;
   DBuf<int> split_off;
   DBuf<double> expn;   // (2 or 4) * expn_stride * NT
+  DBuf<double> mpk;    // packed, scaled M and Mdot of every cell (tc_m2l_warp.cuh)
   size_t expn_stride = 0;  // cells per expansion array: ncell, or ccap in a captured graph
   size_t ccap = 0;
   // lists
@@ -569,23 +571,51 @@ static cudaError_t select_orders(tc_ctx* ctx, TcCells cv, int n, int ntl, const 
   return cudaGetLastError();
 }
 
-// one M2L launch per order class over the class ranges that select_orders wrote: persistent
-// grids (one CTA per SM) taking targets from a counter, the target count read on the device
+// whether the FP64 M2L gives every target a warp (tc_m2l_warp.cuh); the jerks tree always does
+static bool m2l_by_warp(bool jerk, int n) { return jerk || n >= kM2LWarpN; }
+
+// the FP64 M2L of order Q over the target list: persistent grids (one CTA per SM) taking targets
+// from the counter `next`, with `tend` one order class's range of each list
+template <int P, int Q, bool JERK>
+static void m2l_launch(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* ntldev, const int* tbeg,
+                       const int* src, const int* tend, unsigned* next) {
+  cudaStream_t st = ctx->stream;
+  cudaMemsetAsync(next, 0, sizeof(unsigned), st);
+  const int grid = std::max(1, std::min(ntl, ctx->nsm));
+  if (m2l_by_warp(JERK, n)) {
+    k_m2l_warp<Q><<<grid, TcM2LW<Q>::THREADS, TcM2LW<Q>::BYTES, st>>>(ctx->m2l_tl.p, ntl, tbeg, src, cv, ctx->mpk.p,
+                                                                     JERK ? 2 : 1, tc_pk_off(P + 1), TC_NTERM(P),
+                                                                     next, ntldev, tend);
+  } else if constexpr (!JERK) {
+    k_m2l<P, Q><<<grid, tc_m2l_threads<Q>(), (size_t)TcM2LSmem<Q>::TOTAL * sizeof(double), st>>>(
+        ctx->m2l_tl.p, ntl, tbeg, src, cv, ntldev, next, tend);
+  }
+  ctx->launches++;
+}
+
+// packed source expansions of the M2L by warps (nc cells; the buffer is reserved in a capture)
+template <int P, bool JERK>
+static cudaError_t m2l_pack(tc_ctx* ctx, TcCells cv, int n, int nc, const int* ncdev) {
+  if (!m2l_by_warp(JERK, n)) return cudaSuccess;
+  constexpr int NA = JERK ? 2 : 1;
+  cudaError_t e = ctx->mpk.ensure((size_t)nc * NA * tc_pk_off(P + 1));
+  if (e != cudaSuccess) return e;
+  k_m2l_pack<P, NA><<<std::min(nblocks(nc, 8), 148 * 8), 256, 0, ctx->stream>>>(nc, cv.M, cv.Md, ctx->mpk.p, ncdev);
+  ctx->launches++;
+  return cudaGetLastError();
+}
+
+// one M2L launch per order class over the class ranges that select_orders wrote; the target count is
+// read on the device
 template <int P, bool JERK, int I = 0>
-static void m2l_class_launches(tc_ctx* ctx, TcCells cv, int ntl, const unsigned* ntldev, int nc) {
+static void m2l_class_launches(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* ntldev, int nc) {
   using OC = TcOrderClasses<P>;
   using CL = TcClassLaunches<P>;
   if constexpr (I < CL::n) {
     constexpr int F = CL::first(I), E = CL::first(I + 1);  // classes [F, E), at the order of E - 1
-    constexpr int Q = OC::q[E - 1];
-    const size_t smem = (size_t)TcM2LSmem<Q>::TOTAL * sizeof(double);
-    unsigned* next = ctx->d_small + 11;
-    cudaMemsetAsync(next, 0, sizeof(unsigned), ctx->stream);
-    k_m2l<P, Q, JERK><<<ctx->nsm, tc_m2l_threads<Q>(), smem, ctx->stream>>>(
-        ctx->m2l_tl.p, ntl, ctx->cls_rng.p + (size_t)F * nc, ctx->m2l_src2.p, cv, ntldev, next,
-        ctx->cls_rng.p + (size_t)(OC::n + E - 1) * nc);
-    ctx->launches++;
-    m2l_class_launches<P, JERK, I + 1>(ctx, cv, ntl, ntldev, nc);
+    m2l_launch<P, OC::q[E - 1], JERK>(ctx, cv, n, ntl, ntldev, ctx->cls_rng.p + (size_t)F * nc, ctx->m2l_src2.p,
+                                      ctx->cls_rng.p + (size_t)(OC::n + E - 1) * nc, ctx->d_small + 11);
+    m2l_class_launches<P, JERK, I + 1>(ctx, cv, n, ntl, ntldev, nc);
   }
 }
 
@@ -595,8 +625,8 @@ static void set_class_attrs() {
   if constexpr (I < OC::n) {
     constexpr int Q = OC::q[I];
     const int smem = (int)(TcM2LSmem<Q>::TOTAL * sizeof(double));
-    cudaFuncSetAttribute(k_m2l<P, Q, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_m2l<P, Q, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(k_m2l_warp<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcM2LW<Q>::BYTES);
+    cudaFuncSetAttribute(k_m2l<P, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     set_class_attrs<P, I + 1>();
   }
 }
@@ -958,13 +988,13 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
   if (ctx->steps) {
     // time-step pass: no far field (the reference skips M2L when get_steps is set)
   } else if (hs[0] > 0) {
-    const int* m2l_src = ctx->m2l_src.p;
     bool classes = false;
+    if (!mixed) TC_CK((m2l_pack<P, JERK>(ctx, cv, n, ctx->ncell, nullptr)));
     if (prm.selector > 0 && !mixed && TcOrderClasses<P>::n > 1 && ctx->amag_n == n &&
         (prm.selector == 1 || ctx->mlp_ready)) {
       cudaError_t ce = select_orders<P>(ctx, cv, n, (int)hs[0], nullptr, false);
       if (ce != cudaSuccess) return cuda_fail(ctx, ce, "order selection");
-      m2l_class_launches<P, JERK>(ctx, cv, (int)hs[0], nullptr, ctx->ncell);
+      m2l_class_launches<P, JERK>(ctx, cv, n, (int)hs[0], nullptr, ctx->ncell);
       unsigned h[32];
       TC_CK(cudaMemcpyAsync(h, ctx->d_hist, sizeof(h), cudaMemcpyDeviceToHost, st));
       TC_CK(cudaStreamSynchronize(st));
@@ -988,11 +1018,10 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
       k_m2l_mixed<P, JERK><<<hs[0], tc_m2lx_threads<P>(), smem, st>>>(ctx->m2l_tl.p, (int)hs[0], ctx->m2l_start.p,
                                                                         ctx->m2l_src.p, cv);
     } else {
-      size_t smem = (size_t)TcM2LSmem<P>::TOTAL * sizeof(double);
-      k_m2l<P, P, JERK><<<hs[0], tc_m2l_threads<P>(), smem, st>>>(ctx->m2l_tl.p, (int)hs[0], ctx->m2l_start.p,
-                                                                     m2l_src, cv);
+      m2l_launch<P, P, JERK>(ctx, cv, n, (int)hs[0], nullptr, ctx->m2l_start.p, ctx->m2l_src.p, nullptr,
+                             ctx->d_small + 10);
     }
-    ctx->launches++;
+    if (mixed) ctx->launches++;
   }
   if (ctx->events) cudaEventRecord(ctx->ev[4], st);
   // ---- downward, before the near field (the mixed near field reads the far-field
@@ -1134,19 +1163,20 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
   // ---- far field and near field
   TcOut o = out_view(ctx, n, JERK);
   cudaMemsetAsync(ctx->outs.p, 0, sizeof(double) * (size_t)n * (JERK ? 7 : 4), st);
-  cudaMemsetAsync(ctx->d_small + 10, 0, sizeof(unsigned), st);
+  const long long before_m2l = ctx->launches;
+  m2l_pack<P, JERK>(ctx, cv, n, ccap, d_ncell);  // buffer reserved by graph_plan
   if (TcOrderClasses<P>::n < 2) ctx->gselect = false;  // one class: nothing to select
   if (ctx->gselect) {  // per-pair orders (the previous replay left |a| in ctx->amag)
     for (int i = 0; i < TcOrderClasses<P>::n; i++) ctx->gcls_q[i] = TcOrderClasses<P>::q[i];
     ctx->gcls_n = TcOrderClasses<P>::n;
     select_orders<P>(ctx, cv, n, ccap, ctx->d_small, true);
-    m2l_class_launches<P, JERK>(ctx, cv, ccap, ctx->d_small, ccap);
-    L += 4 + TC_MAX_LEVEL + TcClassLaunches<P>::n;
+    m2l_class_launches<P, JERK>(ctx, cv, n, ccap, ctx->d_small, ccap);
     graph_check(ctx, "order selection");
   } else {
-    k_m2l<P, P, JERK><<<ctx->nsm, tc_m2l_threads<P>(), (size_t)TcM2LSmem<P>::TOTAL * sizeof(double), st>>>(
-        ctx->m2l_tl.p, ccap, ctx->m2l_start.p, ctx->m2l_src.p, cv, ctx->d_small, ctx->d_small + 10);
+    m2l_launch<P, P, JERK>(ctx, cv, n, ccap, ctx->d_small, ctx->m2l_start.p, ctx->m2l_src.p, nullptr,
+                           ctx->d_small + 10);
   }
+  L += ctx->launches - before_m2l;
   graph_check(ctx, "M2L");
   graph_event(ctx, 4, st);
   // ---- downward (before the near field: the mixed near field reads the far-field acceleration)
@@ -1208,8 +1238,8 @@ template <int P>
 static void set_m2l_attrs() {
   set_class_attrs<P>();
   size_t smem = (size_t)TcM2LSmem<P>::TOTAL * sizeof(double);
-  cudaFuncSetAttribute(k_m2l<P, P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaFuncSetAttribute(k_m2l<P, P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_m2l_warp<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcM2LW<P>::BYTES);
+  cudaFuncSetAttribute(k_m2l<P, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if constexpr (P <= TC_TC_QMAX) {
     cudaFuncSetAttribute(k_m2l_tc<P, P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcTcSmem<P>::TOTAL);
     cudaFuncSetAttribute(k_m2l_tc<P, P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcTcSmem<P>::TOTAL);
@@ -1219,7 +1249,9 @@ static void set_m2l_attrs() {
   cudaFuncSetAttribute(k_m2l_mixed<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
 }
 
+#ifndef TC_ORDERS
 #define TC_ORDERS(X) X(4) X(6) X(8) X(10) X(12) X(16)
+#endif
 
 static run_fn pick(int p, bool jerk) {
   switch (p) {
@@ -1519,6 +1551,7 @@ tc_status tc_destroy(tc_ctx* ctx) {
   ctx->keys.release(); ctx->keys_alt.release(); ctx->vals.release(); ctx->vals_alt.release(); ctx->hist.release();
   ctx->bod.release(); ctx->bflags.release(); ctx->perm.release(); ctx->outs.release();
   ctx->cint.release(); ctx->cdbl.release(); ctx->csink.release(); ctx->split_off.release(); ctx->expn.release();
+  ctx->mpk.release();
   ctx->front[0].release(); ctx->front[1].release();
   ctx->m2l.release(); ctx->m2l_alt.release(); ctx->p2p.release(); ctx->p2p_alt.release();
   ctx->m2l_start.release(); ctx->m2l_src.release(); ctx->p2p_start.release(); ctx->p2p_src.release();
@@ -1841,7 +1874,7 @@ static void graph_signature(const tc_ctx* c, std::vector<const void*>& s) {
                         c->m2l_alt.p,  c->p2p.p,       c->p2p_alt.p,   c->m2l_start.p, c->m2l_src.p,
                         c->p2p_start.p, c->p2p_src.p,  c->m2l_tl.p,    c->p2p_tl.p,    c->leaves.p,
                         c->judge_idx.p, c->judge_out.p, c->p2p_slots.p, c->bpart.p,    c->tc_bins.p,
-                        c->p2p_s.p,     c->p2p_singles.p, c->p2p_items.p, c->p2p_rows.p,
+                        c->mpk.p,       c->p2p_s.p,     c->p2p_singles.p, c->p2p_items.p, c->p2p_rows.p,
                         c->amag.p,      c->body_scale.p, c->cell_scale.p, c->m2l_src2.p, c->m2l_off.p,
                         c->cell_pn.p,   c->mlp_w.p,      c->cls_rng.p,    c->cell_feat.p};
   s.assign(bufs, bufs + sizeof(bufs) / sizeof(bufs[0]));
@@ -1988,7 +2021,8 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
       ctx->p2p_start.ensure(ccap + 1) || ctx->m2l_src.ensure(ctx->mcap + 1) || ctx->p2p_src.ensure(ctx->pcap + 1) ||
       ctx->m2l_tl.ensure(ccap) || ctx->p2p_tl.ensure(ccap) || ctx->leaves.ensure(ccap) ||
       ctx->expn.ensure(ccap * NT * (jerk ? 4 : 2)) || ctx->bpart.ensure(6 * 148 * 4) ||
-      p2p_reserve(ctx, n, ccap, jerk ? 7 : 4))
+      p2p_reserve(ctx, n, ccap, jerk ? 7 : 4) ||
+      (m2l_by_warp(jerk, n) && ctx->mpk.ensure(ccap * (jerk ? 2 : 1) * tc_pk_off(ctx->prm.p + 1))))
     return;
   if (ctx->prm.selector > 0 &&
       (ctx->cell_pn.ensure(ccap * (ctx->prm.p + 1)) || ctx->cell_scale.ensure(ccap) || ctx->body_scale.ensure(N) ||

@@ -1,4 +1,5 @@
-// Rotation-based O(p^3) M2L in FP64, target-stationary.
+// Rotation-based O(p^3) M2L in FP64, target-stationary: the form of small systems of the top tree
+// (tc_m2l_warp.cuh is all others').
 //
 // Restates M2L_rotate (taichi_with_jerks/kernel_fast_lean.h:1130-1371, one-sided; the
 // top-level mutual form kernel_fast_lean.h:1034-1295 equals two one-sided calls because the
@@ -403,7 +404,7 @@ constexpr int tc_m2l_threads() { return 128 * TcM2LGroups<Q>::G; }
 // evaluation).  One CTA per SM (shared
 // memory), which owns the tensor memory it allocates.  One target per CTA, or, with `next`
 // (a counter zeroed before the launch), a persistent grid whose CTAs take targets in turn.
-template <int P, int Q, bool JERK>
+template <int P, int Q>
 __global__ void __launch_bounds__(tc_m2l_threads<Q>(), 1) k_m2l(const int* __restrict__ tlist, int ntl,
                                                                const int* __restrict__ tstart,
                                                                const int* __restrict__ src, TcCells c,
@@ -447,8 +448,8 @@ __global__ void __launch_bounds__(tc_m2l_threads<Q>(), 1) k_m2l(const int* __res
   // the target's sources: [tstart[t], tstart[t + 1]), or one order class's range of them
   const int s_beg = tstart[t], s_end = tend ? tend[t] : tstart[t + 1];
   const double Xt = c.X[t], Yt = c.Y[t], Zt = c.Z[t];
-  for (int arr = 0; arr < (c.has_sink[t] && s_end > s_beg ? (JERK ? 2 : 1) : 0); arr++) {
-    const double* Mbase = arr ? c.Md : c.M;
+  if (c.has_sink[t] && s_end > s_beg) {
+    const double* Mbase = c.M;
     tc_m2l_zero_warp<Q, QUIRK>(w, twarp);
     for (int b0 = s_beg + grp * 32; b0 < s_end; b0 += 32 * G) {
       int idx = b0 + lane;
@@ -470,7 +471,7 @@ __global__ void __launch_bounds__(tc_m2l_threads<Q>(), 1) k_m2l(const int* __res
     tc_bar_cta();
     // ordered sum over the 32 G lanes of each coefficient: warp per coefficient, lane j adds
     // columns j, j + 32, ... in order, then a fixed butterfly over the lanes
-    double* Lt = (arr ? c.Ld : c.L) + (size_t)t * NTP;
+    double* Lt = c.L + (size_t)t * NTP;
     for (int r = warp; r < NTQ; r += 4 * G) {
       double v = 0.0;
 #pragma unroll

@@ -109,3 +109,22 @@ def test_infinite_velocity_of_a_body_without_mass_in_the_sum():
     out = g.evaluate(x, y, z, m, vx, vy, vz, flags=flags)
     g.close()
     assert all(np.isfinite(out[k]).all() for k in out)
+
+
+@pytest.mark.parametrize("p", [4, 6, 8, 10, 12, 16])
+@pytest.mark.parametrize("n", [2047, 2048])  # the far field's two forms of the top tree
+@pytest.mark.parametrize("variant", [tcb.VARIANT_TOP, tcb.VARIANT_JERKS])
+def test_far_field_of_every_order(p, n, variant):
+    x, y, z, vx, vy, vz, m = _cluster(n, 21)
+    flags = np.full(n, 3, dtype=np.uint8)
+    flags[: n // 3] = 2  # leaves without a sink are no targets
+    o = oracle.evaluate(x, y, z, m, vx, vy, vz, p=p, theta=0.5, ncrit=8, variant=variant, flags=flags)
+    g = tcb.Gravity(p=p, ncrit=8, theta=0.5, variant=variant, direct_below=0)
+    out = g.evaluate(x, y, z, m, vx, vy, vz, flags=flags)
+    assert g.stats()["n_m2l"] == o["stats"]["n_m2l"] > 0
+    g.close()
+    sink = (flags & 1) == 1
+    _close(out, o, ACC, sink)
+    _close(out, o, ("pot",), sink)
+    if variant == tcb.VARIANT_JERKS:
+        _close(out, o, JERK, sink)
