@@ -571,8 +571,8 @@ static cudaError_t select_orders(tc_ctx* ctx, TcCells cv, int n, int ntl, const 
   return cudaGetLastError();
 }
 
-// whether the FP64 M2L gives every target a warp (tc_m2l_warp.cuh); the jerks tree always does
-static bool m2l_by_warp(bool jerk, int n) { return jerk || n >= kM2LWarpN; }
+// whether the FP64 M2L gives every target a warp (tc_m2l_warp.cuh)
+static bool m2l_by_warp(bool jerk, int n) { return (long long)n * (jerk ? 2 : 1) >= kM2LWarpN; }
 
 // the FP64 M2L of order Q over the target list: persistent grids (one CTA per SM) taking targets
 // from the counter `next`, with `tend` one order class's range of each list
@@ -580,17 +580,25 @@ template <int P, int Q, bool JERK>
 static void m2l_launch(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* ntldev, const int* tbeg,
                        const int* src, const int* tend, unsigned* next) {
   cudaStream_t st = ctx->stream;
-  cudaMemsetAsync(next, 0, sizeof(unsigned), st);
   const int grid = std::max(1, std::min(ntl, ctx->nsm));
-  if (m2l_by_warp(JERK, n)) {
-    k_m2l_warp<Q><<<grid, TcM2LW<Q>::THREADS, TcM2LW<Q>::BYTES, st>>>(ctx->m2l_tl.p, ntl, tbeg, src, cv, ctx->mpk.p,
-                                                                     JERK ? 2 : 1, tc_pk_off(P + 1), TC_NTERM(P),
-                                                                     next, ntldev, tend);
-  } else if constexpr (!JERK) {
-    k_m2l<P, Q><<<grid, tc_m2l_threads<Q>(), (size_t)TcM2LSmem<Q>::TOTAL * sizeof(double), st>>>(
-        ctx->m2l_tl.p, ntl, tbeg, src, cv, ntldev, next, tend);
+  const bool by_warp = m2l_by_warp(JERK, n);
+  for (int arr = 0; arr < (JERK && !by_warp ? 2 : 1); arr++) {
+    cudaMemsetAsync(next, 0, sizeof(unsigned), st);
+    if (by_warp) {
+      k_m2l_warp<Q><<<grid, TcM2LW<Q>::THREADS, TcM2LW<Q>::BYTES, st>>>(ctx->m2l_tl.p, ntl, tbeg, src, cv, ctx->mpk.p,
+                                                                       JERK ? 2 : 1, tc_pk_off(P + 1), TC_NTERM(P),
+                                                                       next, ntldev, tend);
+    } else {
+      TcCells ca = cv;  // Mdot -> Ldot as a launch of its own
+      if (arr) {
+        ca.M = cv.Md;
+        ca.L = cv.Ld;
+      }
+      k_m2l<P, Q><<<grid, tc_m2l_threads<Q>(), (size_t)TcM2LSmem<Q>::TOTAL * sizeof(double), st>>>(
+          ctx->m2l_tl.p, ntl, tbeg, src, ca, ntldev, next, tend);
+    }
+    ctx->launches++;
   }
-  ctx->launches++;
 }
 
 // packed source expansions of the M2L by warps (nc cells; the buffer is reserved in a capture)
@@ -835,11 +843,23 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
     if (g > 148 * 16) g = 148 * 16;
     k_p2m_leaves<P, JERK><<<g, kP2MWarps * 32, 0, st>>>(ctx->ncell, b, cv);
   }
-  for (int l = maxl; l >= 0; l--) {
-    int cnt = ctx->lv.count[l];
-    int g = nblocks(cnt, TcTransW<P>::W);
-    if (g > 148 * 16) g = 148 * 16;
-    k_upward_level<P, JERK><<<g, TcTransW<P>::W * 32, 0, st>>>(l, b, cv, d_start, d_count, ctx->d_err);
+  // inner cells: balls two levels at a time, then M2M level by level (the deepest level has leaves only)
+  for (int l = (maxl - 1) & ~1; l >= 0; l -= 2) {
+    const int cnt = ctx->lv.count[l] + ctx->lv.count[l + 1];
+    if (cnt <= kFewCells)
+      k_inner_balls_few<<<cnt, 256, 0, st>>>(l, b, cv, d_start, d_count, ctx->d_err);
+    else
+      k_inner_balls<<<std::min(nblocks(cnt, kUpWarps), 148 * 16), kUpWarps * 32, 0, st>>>(l, b, cv, d_start, d_count,
+                                                                                          ctx->d_err);
+    ctx->launches++;
+  }
+  for (int l = maxl - 1; l >= 0; l--) {
+    const int cnt = ctx->lv.count[l];
+    if (cnt <= kFewCells)
+      k_m2m_few<P, JERK><<<cnt, 256, TcM2MFew<P, JERK>::BYTES, st>>>(l, cv, d_start, d_count);
+    else
+      k_m2m_level<P, JERK><<<std::min(nblocks(cnt, TcTransW<P>::W), 148 * 16), TcTransW<P>::W * 32, 0, st>>>(
+          l, cv, d_start, d_count);
   }
   if (ctx->events) cudaEventRecord(ctx->ev[2], st);
   // ---- traversal, list sort and per-target offsets (lists of the acceptance test `mac` over the
@@ -1121,9 +1141,17 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
     g = std::min(nblocks(ccap, kP2MWarps), 148 * 16);
     k_p2m_leaves<P, JERK><<<g, kP2MWarps * 32, 0, st>>>(ccap, b, cv, ctx->d_lv);
   }
-  for (int l = TC_MAX_LEVEL; l >= 0; l--)
-    k_upward_level<P, JERK><<<148 * 16, TcTransW<P>::W * 32, 0, st>>>(l, b, cv, d_start, d_count, ctx->d_err);
-  L += 2 + TC_MAX_LEVEL + 1;
+  for (int l = (TC_MAX_LEVEL - 1) & ~1; l >= 0; l -= 2) {  // each form returns at once where the other applies
+    k_inner_balls_few<<<kFewCells, 256, 0, st>>>(l, b, cv, d_start, d_count, ctx->d_err);
+    k_inner_balls<<<148 * 16, kUpWarps * 32, 0, st>>>(l, b, cv, d_start, d_count, ctx->d_err);
+    L += 2;
+  }
+  for (int l = TC_MAX_LEVEL - 1; l >= 0; l--) {
+    k_m2m_few<P, JERK><<<kFewCells, 256, TcM2MFew<P, JERK>::BYTES, st>>>(l, cv, d_start, d_count);
+    k_m2m_level<P, JERK><<<148 * 16, TcTransW<P>::W * 32, 0, st>>>(l, cv, d_start, d_count);
+    L += 2;
+  }
+  L += 2;
   graph_check(ctx, "upward pass");
   graph_event(ctx, 2, st);
   // ---- traversal
@@ -1244,6 +1272,9 @@ static void set_m2l_attrs() {
     cudaFuncSetAttribute(k_m2l_tc<P, P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcTcSmem<P>::TOTAL);
     cudaFuncSetAttribute(k_m2l_tc<P, P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcTcSmem<P>::TOTAL);
   }
+  cudaFuncSetAttribute(k_m2m_few<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcM2MFew<P, true>::BYTES);
+  cudaFuncSetAttribute(k_m2m_few<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)TcM2MFew<P, false>::BYTES);
   size_t smx = (size_t)TcM2LMixSmem<P>::BYTES;
   cudaFuncSetAttribute(k_m2l_mixed<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
   cudaFuncSetAttribute(k_m2l_mixed<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
@@ -1764,7 +1795,7 @@ static tc_status evaluate_impl(tc_ctx* ctx, int n, const double* x, const double
       int nb = 148 * 4;
       TC_CK(ctx->bpart.ensure(6 * nb));
       k_bounds_partial<<<nb, 256, 0, st>>>(n, dx, dy, dz, dm, ctx->bpart.p, ctx->d_err);
-      k_bounds_final<<<1, 1, 0, st>>>(nb, ctx->bpart.p, ctx->d_root, ctx->prm.use_shift, ctx->prm.shift_u[0],
+      k_bounds_final<<<1, kBoundsThreads, 0, st>>>(nb, ctx->bpart.p, ctx->d_root, ctx->prm.use_shift, ctx->prm.shift_u[0],
                                       ctx->prm.shift_u[1], ctx->prm.shift_u[2]);
       k_morton<<<nblocks(n, 256), 256, 0, st>>>(n, dx, dy, dz, ctx->d_root, ctx->keys.p, ctx->vals.p);
       ctx->launches += 4 + radix_sort(ctx->keys.p, ctx->vals.p, ctx->keys_alt.p, ctx->vals_alt.p, n, 63, ctx->hist.p, st);
@@ -1932,7 +1963,7 @@ static void graph_issue(tc_ctx* ctx, int n, const double* const* in, const unsig
   TcBodies b = bodies_view(ctx, n, jerk);
   const int nb = 148 * 4;
   k_bounds_partial<<<nb, 256, 0, st>>>(n, dx, dy, dz, dm, ctx->bpart.p, ctx->d_err);
-  k_bounds_final<<<1, 1, 0, st>>>(nb, ctx->bpart.p, ctx->d_root, ctx->prm.use_shift, ctx->prm.shift_u[0],
+  k_bounds_final<<<1, kBoundsThreads, 0, st>>>(nb, ctx->bpart.p, ctx->d_root, ctx->prm.use_shift, ctx->prm.shift_u[0],
                                   ctx->prm.shift_u[1], ctx->prm.shift_u[2]);
   k_morton<<<nblocks(n, 256), 256, 0, st>>>(n, dx, dy, dz, ctx->d_root, ctx->keys.p, ctx->vals.p);
   L += 4 + radix_sort(ctx->keys.p, ctx->vals.p, ctx->keys_alt.p, ctx->vals_alt.p, n, 63, ctx->hist.p, st);

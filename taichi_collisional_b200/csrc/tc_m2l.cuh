@@ -1,5 +1,5 @@
-// Rotation-based O(p^3) M2L in FP64, target-stationary: the form of small systems of the top tree
-// (tc_m2l_warp.cuh is all others').
+// Rotation-based O(p^3) M2L in FP64, target-stationary: the form of small systems (tc_m2l_warp.cuh is
+// the large ones').  One expansion a launch: Mdot goes as a launch of its own.
 //
 // Restates M2L_rotate (taichi_with_jerks/kernel_fast_lean.h:1130-1371, one-sided; the
 // top-level mutual form kernel_fast_lean.h:1034-1295 equals two one-sided calls because the

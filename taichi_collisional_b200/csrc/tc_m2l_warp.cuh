@@ -31,9 +31,10 @@
 
 namespace tc {
 
-// below this many bodies there are too few targets for a warp each; k_m2l's four warps per batch of
-// pairs then finish sooner
-constexpr int kM2LWarpN = 2048;
+// below this many bodies times expansions there are too few targets (about one per 15 bodies) for the
+// GPU's warps, and k_m2l's four warps per batch of pairs finish sooner (top tree, p = 8: N = 16,384
+// 0.125 ms against 0.18; N = 131,072 1.48 against 1.27)
+constexpr int kM2LWarpN = 65536;
 
 // ---- packed source expansions: degree d at tc_pk_off(d), (2 d + 1) rounded up to 4 doubles
 __host__ __device__ constexpr int tc_pk_width(int d) { return (2 * d + 1 + 3) / 4 * 4; }

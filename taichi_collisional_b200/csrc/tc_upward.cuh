@@ -1,6 +1,6 @@
 // Upward pass on the device: the balls of every leaf (one launch), P2M of every leaf (one
-// launch), then one launch per tree level (deepest first) for the inner cells, one warp per
-// cell.  Restates upwardPass (traverse_eager.h:9-34) with MINIBALL: each cell's expansion centre
+// launch), the balls of the inner cells two tree levels at a time (deepest first), then M2M level by
+// level.  Levels of many cells take a warp per cell, levels of few cells a CTA per cell.  Restates upwardPass (traverse_eager.h:9-34) with MINIBALL: each cell's expansion centre
 // and radius are the smallest ball enclosing its bodies (leaf, kernel_fast_lean.h:707-737)
 // or, for an inner cell, the bodies of its leaf children plus 64 t-design points around
 // every grandchild (:833-892); R = r_ball + 1e-6.  Then P2M (:745-781) for leaves and M2M
@@ -8,6 +8,7 @@
 // 769-817, :950-998).
 #pragma once
 #include "tc_harmonics.cuh"
+#include "tc_tree.cuh"
 
 namespace tc {
 
@@ -188,10 +189,24 @@ __device__ __forceinline__ void tc_point_td(const TcPointSet& ps, int idx, const
   }
 }
 
+// not converged: grow the ball to enclose every point and flag it
+__device__ void tc_mb_enclose(const TcPointSet& ps, const TcBodies& b, const TcCells& cl, const double* td,
+                              const double* c, double* r2, unsigned int* err) {
+  const int lane = threadIdx.x & 31;
+  double mx = 0;
+  for (int i = lane; i < ps.total; i += 32) {
+    double p[3];
+    tc_point_td(ps, i, b, cl, td, p);
+    mx = fmax(mx, tc_d2(p, c));
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  *r2 = fmax(*r2, mx);
+  if (lane == 0) tc_set_err(err, TC_EBIT_MINIBALL);
+}
+
 // every lane of the warp ends with the same (c, r2)
 __device__ void tc_warp_miniball(const TcPointSet& ps, const TcBodies& b, const TcCells& cl, const double* td,
                                  double* c, double* r2, unsigned int* err) {
-  int lane = threadIdx.x & 31;
   double s[4][3];
   int ns = 1;
   tc_point_td(ps, 0, b, cl, td, s[0]);
@@ -208,16 +223,7 @@ __device__ void tc_warp_miniball(const TcPointSet& ps, const TcBodies& b, const 
     if (!tc_mb_small(s, ns, q, c, r2)) break;
     if (!(*r2 > old)) return;  // no growth: the ball is final (the reference's stop rule)
   }
-  // not converged: grow the ball to enclose every point and flag it
-  double mx = 0;
-  for (int i = lane; i < ps.total; i += 32) {
-    double p[3];
-    tc_point_td(ps, i, b, cl, td, p);
-    mx = fmax(mx, tc_d2(p, c));
-  }
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  *r2 = fmax(*r2, mx);
-  if (lane == 0) tc_set_err(err, TC_EBIT_MINIBALL);
+  tc_mb_enclose(ps, b, cl, td, c, r2, err);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -450,6 +456,76 @@ __device__ void tc_m2m_warp(int ci, const TcCells& c, cd* G, cd* SM, cd* SMd) {
   }
 }
 
+// The same sums, a warp per child: at the levels of few cells the latency of one warp that takes the
+// children in turn is the launch's time (N = 2,000, p = 8: 130 us a level with the ball search, 7 levels).
+// The children's contributions meet in shared memory and are added in child order, as tc_m2m_warp does.
+constexpr int kFewCells = 148 * 4;  // levels of at most this many inner candidates get a CTA per cell
+template <int P, bool JERK>
+struct TcM2MFew {
+  static constexpr int NT = (P + 1) * (P + 1), NOUT = (P + 1) * (P + 2) / 2;
+  static constexpr size_t BYTES = sizeof(cd) * 8 * ((JERK ? 3 : 2) * NT + (JERK ? 2 : 1) * NOUT);
+};
+template <int P, bool JERK>
+__global__ void __launch_bounds__(256) k_m2m_few(int l, TcCells c, const int* __restrict__ lv_start,
+                                                 const int* __restrict__ lv_count) {
+  constexpr int NT = TcM2MFew<P, JERK>::NT, NOUT = TcM2MFew<P, JERK>::NOUT;
+  extern __shared__ __align__(16) unsigned char tc_few_smem[];
+  cd* base = reinterpret_cast<cd*>(tc_few_smem);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  cd* G = base + w * NT;
+  cd* SM = base + 8 * NT + w * NT;
+  cd* SMd = JERK ? base + 16 * NT + w * NT : nullptr;
+  cd* part = base + (JERK ? 24 : 16) * NT;  // [child][NOUT], then the same of Mdot
+  const int cnt = lv_count[l], st = lv_start[l];
+  if (cnt > kFewCells) return;
+  for (int q = blockIdx.x; q < cnt; q += gridDim.x) {
+    const int ci = st + q;
+    const int nch = c.nchild[ci], ch = c.child[ci] + w;
+    if (nch == 0) continue;
+    if (w < nch) {
+      const double* Mc = c.M + (size_t)ch * NT;
+      const double* Mdc = JERK ? c.Md + (size_t)ch * NT : nullptr;
+      for (int i = lane; i < NT; i += 32) {
+        int n = 0;
+        while ((n + 1) * (n + 1) <= i) n++;
+        SM[i] = tc_r2c(Mc, n, i - n * n - n);
+        if (JERK) SMd[i] = tc_r2c(Mdc, n, i - n * n - n);
+      }
+      tc_warp_gnm_smem<P>(c.X[ch] - c.X[ci], c.Y[ch] - c.Y[ci], c.Z[ch] - c.Z[ci], G);  // ends with __syncwarp
+      for (int o = lane; o < NOUT; o += 32) {
+        int n = 0;
+        while ((n + 1) * (n + 2) / 2 <= o) n++;
+        const int m = o - n * (n + 1) / 2;
+        cd s = mk(0, 0), sd = mk(0, 0);
+        for (int kk = 0; kk <= n; kk++) {
+          const int lo = max(-kk, m - n + kk), hi = min(kk, m + n - kk);
+          const int nn = n - kk, b0 = nn * nn + nn + m;  // source (n - kk, m - l)
+          for (int j = lo; j <= hi; j++) {
+            cd g = G[kk * kk + kk + j];
+            s += SM[b0 - j] * g;
+            if (JERK) sd += SMd[b0 - j] * g;
+          }
+        }
+        part[w * NOUT + o] = s;
+        if (JERK) part[(8 + w) * NOUT + o] = sd;
+      }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < (JERK ? 2 : 1) * NOUT; k += blockDim.x) {
+      const int o = k % NOUT, a = k / NOUT;
+      int n = 0;
+      while ((n + 1) * (n + 2) / 2 <= o) n++;
+      const int m = o - n * (n + 1) / 2, is = n * n + n;
+      cd acc = mk(0, 0);
+      for (int x = 0; x < nch; x++) acc += part[(8 * a + x) * NOUT + o];
+      double* M = (a ? c.Md : c.M) + (size_t)ci * NT;
+      M[is + m] = acc.x;
+      if (m > 0) M[is - m] = acc.y;
+    }
+    __syncthreads();
+  }
+}
+
 // warps per block of the M2M and L2L level kernels (three NT-complex arrays per warp in
 // static shared memory, at most 48 KB)
 template <int P>
@@ -473,79 +549,244 @@ __device__ __forceinline__ void tc_load_tdesign(double* s_td) {
   __syncthreads();
 }
 
-// one warp: expansion centre, radius and has_sink of cell ci
+// point set of the ball of an inner cell: the bodies of its leaf children, 64 points around each
+// grandchild
+__device__ __forceinline__ void tc_inner_points(int ci, const TcCells& c, TcPointSet& ps) {
+  const int nch = c.nchild[ci];
+  ps.leaf = 0;
+  ps.nseg = nch;
+  int tot = 0;
+  for (int s = 0; s < nch; s++) {
+    const int ch = c.child[ci] + s;
+    ps.seg_start[s] = tot;
+    if (c.nchild[ch] == 0) {
+      ps.seg_kind[s] = 0;
+      ps.seg_a[s] = c.begin[ch];
+      tot += c.nbody[ch];
+    } else {
+      ps.seg_kind[s] = 1;
+      ps.seg_a[s] = c.child[ch];
+      tot += 64 * c.nchild[ch];
+    }
+  }
+  ps.seg_start[nch] = tot;
+  ps.total = tot;
+}
+
+// one warp: expansion centre and radius of cell ci
 __device__ void tc_cell_ball(int ci, const TcBodies& b, TcCells& c, const double* s_td, unsigned int* err) {
   int lane = threadIdx.x & 31;
   TcPointSet ps;
-  int nch = c.nchild[ci];
-  bool sink = false;
-  if (nch == 0) {
+  if (c.nchild[ci] == 0) {
     ps.leaf = 1;
     ps.seg_a[0] = c.begin[ci];
     ps.total = c.nbody[ci];
-    for (int i = c.begin[ci] + lane; i < c.begin[ci] + c.nbody[ci]; i += 32) sink |= (b.flags[i] & 1) != 0;
   } else {
-    ps.leaf = 0;
-    ps.nseg = nch;
-    int tot = 0;
-    for (int s = 0; s < nch; s++) {
-      int ch = c.child[ci] + s;
-      ps.seg_start[s] = tot;
-      sink |= c.has_sink[ch] != 0;
-      if (c.nchild[ch] == 0) {
-        ps.seg_kind[s] = 0;
-        ps.seg_a[s] = c.begin[ch];
-        tot += c.nbody[ch];
-      } else {
-        ps.seg_kind[s] = 1;
-        ps.seg_a[s] = c.child[ch];
-        tot += 64 * c.nchild[ch];
-      }
-    }
-    ps.seg_start[nch] = tot;
-    ps.total = tot;
+    tc_inner_points(ci, c, ps);
   }
-  sink = __any_sync(0xffffffffu, sink);
   double cc[3], r2;
   tc_warp_miniball(ps, b, c, s_td, cc, &r2, err);
   if (lane == 0) {
     c.X[ci] = cc[0]; c.Y[ci] = cc[1]; c.Z[ci] = cc[2];
     c.R[ci] = sqrt(r2) + 1e-6;
-    c.has_sink[ci] = sink;
   }
   __syncwarp();
 }
 
-// balls of every leaf (they depend on the leaf's own bodies only)
+// Balls of every leaf (they depend on the leaf's own bodies only), and has_sink of every cell: a leaf
+// with a sink marks its ancestors up to the first one already marked (cells start unmarked).
 __global__ void __launch_bounds__(kUpWarps * 32) k_leaf_balls(int ncell, const TcBodies b, TcCells c,
                                                               unsigned int* err, const TcLevels* lvd = nullptr) {
   __shared__ double s_td[193];
   tc_load_tdesign(s_td);
   if (lvd) ncell = lvd->ncell;  // device-sized launch (graph): the cell count of this tree
-  int w = threadIdx.x >> 5;
-  for (int ci = blockIdx.x * kUpWarps + w; ci < ncell; ci += gridDim.x * kUpWarps)
-    if (c.nchild[ci] == 0) tc_cell_ball(ci, b, c, s_td, err);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int ci = blockIdx.x * kUpWarps + w; ci < ncell; ci += gridDim.x * kUpWarps) {
+    if (c.nchild[ci] != 0) continue;
+    tc_cell_ball(ci, b, c, s_td, err);
+    bool sink = false;
+    for (int i = c.begin[ci] + lane; i < c.begin[ci] + c.nbody[ci]; i += 32) sink |= (b.flags[i] & 1) != 0;
+    if (__any_sync(0xffffffffu, sink) && lane == 0) {
+      volatile uint8_t* hs = c.has_sink;
+      for (int p = ci; p >= 0 && !hs[p]; p = c.parent[p]) hs[p] = 1;
+    }
+  }
 }
 
-// inner cells of level l: ball over the children's points, then M2M from the children
+// Balls of the inner cells of levels l and l + 1.  A ball reads the balls of grandchildren (or bodies),
+// so two levels have no dependence on each other and go together: half the launches of the chain.
+// Many cells: a warp each.
+__global__ void __launch_bounds__(kUpWarps * 32) k_inner_balls(int l, const TcBodies b, TcCells c,
+                                                               const int* __restrict__ lv_start,
+                                                               const int* __restrict__ lv_count, unsigned int* err) {
+  __shared__ double s_td[193];
+  const int cnt = lv_count[l] + lv_count[l + 1], st = lv_start[l];  // the two levels are contiguous
+  if (cnt <= kFewCells) return;
+  tc_load_tdesign(s_td);
+  const int w = threadIdx.x >> 5;
+  for (int k = blockIdx.x * kUpWarps + w; k < cnt; k += gridDim.x * kUpWarps)
+    if (c.nchild[st + k] != 0) tc_cell_ball(st + k, b, c, s_td, err);
+}
+
+// Few cells: a CTA each.  The farthest-point search, most of the work, goes over all 256 threads; the
+// exact small solver stays one warp's.  The same points with the same arithmetic and the same choice
+// among equals as the warp's search (which only skips groups that cannot win), so the same ball.
+constexpr int kFewBodies = 512;  // bodies of leaf children kept in shared memory
+__global__ void __launch_bounds__(256) k_inner_balls_few(int l, const TcBodies b, TcCells c,
+                                                         const int* __restrict__ lv_start,
+                                                         const int* __restrict__ lv_count, unsigned int* err) {
+  __shared__ double s_td[193];
+  __shared__ TcPointSet ps;
+  __shared__ double sgx[64], sgy[64], sgz[64], sgr[64];                      // grandchildren
+  __shared__ double sbx[kFewBodies], sby[kFewBodies], sbz[kFewBodies];       // bodies
+  __shared__ int gbase[64], bbase[9], bseg[9], klen[8], ng, nseg0, nbod;
+  __shared__ double red_e[8], s_c[4];
+  __shared__ int red_i[8], s_go;
+  const int cnt = lv_count[l] + lv_count[l + 1], st = lv_start[l];
+  if (cnt > kFewCells) return;
+  tc_load_tdesign(s_td);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int k = blockIdx.x; k < cnt; k += gridDim.x) {
+    const int ci = st + k;
+    if (c.nchild[ci] == 0) continue;
+    __syncthreads();
+    if (threadIdx.x < c.nchild[ci]) {
+      const int ch = c.child[ci] + threadIdx.x, n = c.nchild[ch];
+      ps.seg_kind[threadIdx.x] = n > 0;
+      ps.seg_a[threadIdx.x] = n ? c.child[ch] : c.begin[ch];
+      klen[threadIdx.x] = n ? 64 * n : c.nbody[ch];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      ps.leaf = 0;
+      ps.nseg = c.nchild[ci];
+      ps.total = 0;
+      ng = nseg0 = nbod = 0;
+      for (int s = 0; s < ps.nseg; s++) {
+        const int len = klen[s];
+        ps.seg_start[s] = ps.total;
+        ps.total += len;
+        ps.seg_start[s + 1] = ps.total;
+        if (ps.seg_kind[s] == 0) {  // bodies: their place in the shared list, their place among the points
+          bbase[nseg0] = nbod;
+          bseg[nseg0++] = s;
+          nbod += len;
+        } else {
+          for (int g = 0; g < (len >> 6); g++) gbase[ng++] = ps.seg_start[s] + (g << 6);
+        }
+      }
+      bbase[nseg0] = nbod;
+    }
+    __syncthreads();
+    const bool fits = nbod <= kFewBodies;
+    if (threadIdx.x < ng) {
+      int s = 0;
+      while (gbase[threadIdx.x] >= ps.seg_start[s + 1]) s++;
+      const int g = ps.seg_a[s] + ((gbase[threadIdx.x] - ps.seg_start[s]) >> 6);
+      sgx[threadIdx.x] = c.X[g]; sgy[threadIdx.x] = c.Y[g]; sgz[threadIdx.x] = c.Z[g]; sgr[threadIdx.x] = c.R[g];
+    }
+    if (fits)
+      for (int i = threadIdx.x; i < nbod; i += blockDim.x) {
+        int q = 0;
+        while (i >= bbase[q + 1]) q++;
+        const int j = ps.seg_a[bseg[q]] + i - bbase[q];
+        sbx[i] = b.x[j]; sby[i] = b.y[j]; sbz[i] = b.z[j];
+      }
+    double sup[4][3], cc[3], r2 = 0;  // warp 0: the support set
+    int ns = 1;
+    if (w == 0) {
+      tc_point_td(ps, 0, b, c, s_td, sup[0]);
+      cc[0] = sup[0][0]; cc[1] = sup[0][1]; cc[2] = sup[0][2];
+      if (lane == 0) { s_c[0] = cc[0]; s_c[1] = cc[1]; s_c[2] = cc[2]; s_c[3] = 0; }
+    }
+    bool grow = true;
+    for (int it = 0; it < 512; it++) {
+      __syncthreads();
+      const double ctr[3] = {s_c[0], s_c[1], s_c[2]}, rr = s_c[3];
+      double be = 0;
+      int bi = 0x7fffffff;
+      for (int i = threadIdx.x; i < nbod; i += blockDim.x) {
+        int q = 0;
+        while (i >= bbase[q + 1]) q++;
+        double p[3];
+        if (fits) {
+          p[0] = sbx[i]; p[1] = sby[i]; p[2] = sbz[i];
+        } else {
+          const int j = ps.seg_a[bseg[q]] + i - bbase[q];
+          p[0] = b.x[j]; p[1] = b.y[j]; p[2] = b.z[j];
+        }
+        const double e = tc_d2(p, ctr) - rr;
+        const int id = ps.seg_start[bseg[q]] + i - bbase[q];
+        if (e > be || (e == be && e > 0 && id < bi)) { be = e; bi = id; }
+      }
+      for (int i = threadIdx.x; i < 64 * ng; i += blockDim.x) {
+        const int g = i >> 6, t = i & 63;
+        const double R = sgr[g];
+        const double p[3] = {sgx[g] + R * s_td[3 * t], sgy[g] + R * s_td[3 * t + 1], sgz[g] + R * s_td[3 * t + 2]};
+        const double e = tc_d2(p, ctr) - rr;
+        const int id = gbase[g] + t;
+        if (e > be || (e == be && e > 0 && id < bi)) { be = e; bi = id; }
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double oe = __shfl_xor_sync(0xffffffffu, be, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (oe > be || (oe == be && oi < bi)) { be = oe; bi = oi; }
+      }
+      if (lane == 0) { red_e[w] = be; red_i[w] = bi; }
+      __syncthreads();
+      if (w == 0) {
+        be = red_e[lane & 7];
+        bi = red_i[lane & 7];
+        for (int o = 4; o > 0; o >>= 1) {
+          const double oe = __shfl_xor_sync(0xffffffffu, be, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (oe > be || (oe == be && oi < bi)) { be = oe; bi = oi; }
+        }
+        int go = 1;  // 0: final, 1: on, 2: not converged
+        if (bi == 0x7fffffff || be <= r2 * 1e-15) {
+          go = 0;
+        } else {
+          double q[3];
+          tc_point_td(ps, bi, b, c, s_td, q);
+          const double old = r2;
+          if (!tc_mb_small(sup, ns, q, cc, &r2)) go = 2;
+          else if (!(r2 > old)) go = 0;
+        }
+        if (lane == 0) {
+          s_c[0] = cc[0]; s_c[1] = cc[1]; s_c[2] = cc[2]; s_c[3] = r2;
+          s_go = go;
+        }
+      }
+      __syncthreads();
+      if (s_go != 1) {
+        grow = s_go == 2;
+        break;
+      }
+    }
+    if (w == 0) {
+      if (grow) tc_mb_enclose(ps, b, c, s_td, cc, &r2, err);
+      if (lane == 0) {
+        c.X[ci] = cc[0]; c.Y[ci] = cc[1]; c.Z[ci] = cc[2];
+        c.R[ci] = sqrt(r2) + 1e-6;
+      }
+    }
+  }
+}
+
+// M2M into the inner cells of level l from their children, a warp per cell
 template <int P, bool JERK>
-__global__ void __launch_bounds__(TcTransW<P>::W * 32) k_upward_level(int l, const TcBodies b, TcCells c,
-                                                                      const int* __restrict__ lv_start,
-                                                                      const int* __restrict__ lv_count,
-                                                                      unsigned int* err) {
+__global__ void __launch_bounds__(TcTransW<P>::W * 32) k_m2m_level(int l, TcCells c, const int* __restrict__ lv_start,
+                                                                   const int* __restrict__ lv_count) {
   constexpr int W = TcTransW<P>::W, NT = (P + 1) * (P + 1);
   __shared__ cd sG[W][NT];
   __shared__ cd sM[W][NT];
   __shared__ cd sMd[W][JERK ? NT : 1];
-  __shared__ double s_td[193];
-  tc_load_tdesign(s_td);
-  int w = threadIdx.x >> 5;
-  int cnt = lv_count[l], st = lv_start[l];
+  const int w = threadIdx.x >> 5;
+  const int cnt = lv_count[l], st = lv_start[l];
+  if (cnt <= kFewCells) return;
   for (int k = blockIdx.x * W + w; k < cnt; k += gridDim.x * W) {
-    int ci = st + k;
-    if (c.nchild[ci] == 0) continue;
-    tc_cell_ball(ci, b, c, s_td, err);
-    tc_m2m_warp<P, JERK>(ci, c, sG[w], sM[w], sMd[w]);
+    if (c.nchild[st + k] == 0) continue;
+    tc_m2m_warp<P, JERK>(st + k, c, sG[w], sM[w], sMd[w]);
     __syncwarp();
   }
 }
