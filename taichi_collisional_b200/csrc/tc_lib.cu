@@ -209,6 +209,7 @@ struct tc_ctx {
   int gjudge_nt = 0;
   long long glaunches = 0;
   int gsbits = 1;
+  int glist_cells = 0;  // cells the graph's list bitmaps cover
   std::string gfail;  // why the last capture was abandoned (empty: captured)
   std::vector<const void*> gsig;  // buffers and capacities baked into the captured graph
   double gstep_dt = 0.0;          // the graph being planned holds a leapfrog step of this dt
@@ -458,6 +459,20 @@ static TcP2PWork p2p_plan(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigne
   W.slots = ctx->p2p_slots.p;
   W.shared = p2p_shared(ctx);
   return W;
+}
+
+// per-target offsets and ordered sources of one list from the traversal's counts (in tgt_start) and keys;
+// hist: scan scratch.  bits: cells the bitmap covers
+static void list_build(tc_ctx* ctx, const unsigned long long* keys, size_t n, int ncell, int bits, int sbits,
+                       int* tgt_start, int* src, const unsigned long long* ndev, const int* ncdev) {
+  cudaStream_t st = ctx->stream;
+  ctx->launches += excl_scan(reinterpret_cast<uint32_t*>(tgt_start), ncell + 1, ctx->hist.p, st);
+  k_list_scatter<<<(int)std::min<size_t>(nblocks((long long)n, 256) + 1, 148 * 16), 256, 0, st>>>(
+      keys, n, ncell, bits, sbits, tgt_start, src, ctx->d_err, ndev, ncdev);
+  const size_t smem = ((size_t)bits + 31) / 32 * 4;
+  const int resident = std::max(1, std::min(16, (int)(220 * 1024 / (smem + 1024))));
+  k_list_order<<<std::min(ncell, 148 * resident), kListThreads, smem, st>>>(ncell, bits, tgt_start, src, ncdev);
+  ctx->launches += 2;
 }
 
 // the near field itself: a persistent grid over the items, then the split rows folded
@@ -722,7 +737,7 @@ static tc_status train_selector(tc_ctx* ctx, int nsamples, int iters, unsigned l
   TcBodies b = bodies_view(ctx, ctx->n, jerk);
   const int K = (int)std::min<unsigned long long>((unsigned long long)nsamples, ctx->n_m2l);
   if (K < 16) return TC_ERR_ARG;
-  // the fixed-order evaluation left the sorted (target, source) list in m2l
+  // the fixed-order evaluation left the per-target source lists in m2l_start and m2l_src
   std::vector<long long> idx(K);
   std::mt19937_64 rng(seed);
   std::uniform_int_distribution<unsigned long long> U(0, ctx->n_m2l - 1);
@@ -740,7 +755,7 @@ static tc_status train_selector(tc_ctx* ctx, int nsamples, int iters, unsigned l
   TC_CK(cudaMalloc((void**)&d_feat, (size_t)K * kMlpIn * sizeof(float)));
   TC_CK(cudaMalloc((void**)&d_lab, (size_t)K * OC::n * sizeof(float)));
   TC_CK(cudaMemcpyAsync(d_idx, idx.data(), K * sizeof(long long), cudaMemcpyHostToDevice, st));
-  k_gather_pairs<<<(K + 255) / 256, 256, 0, st>>>(K, ctx->m2l.p, d_idx, ctx->sbits, pt, ps);
+  k_gather_pairs<<<(K + 255) / 256, 256, 0, st>>>(K, nc, ctx->m2l_start.p, ctx->m2l_src.p, d_idx, pt, ps);
   k_cell_pn<P><<<nblocks(nc, 128), 128, 0, st>>>(nc, cv.M, ctx->cell_pn.p);
   TcClassPairs<P, 0>::run(K, pt, ps, cv, Lcls, st);
   k_pair_eval<P><<<K, 128, 0, st>>>(K, OC::n, pt, ps, b, cv, ctx->cell_pn.p, Lcls, d_lab);
@@ -882,13 +897,18 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
     ctx->pcap = ctx->p2p.n;
     ctx->fcap = ctx->front[0].n < ctx->front[1].n ? ctx->front[0].n : ctx->front[1].n;
     TC_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), st));
+    TC_CK(ctx->m2l_start.ensure(ctx->ncell + 1));
+    TC_CK(ctx->p2p_start.ensure(ctx->ncell + 1));
+    TC_CK(cudaMemsetAsync(ctx->m2l_start.p, 0, sizeof(int) * ((size_t)ctx->ncell + 1), st));  // pairs per target
+    TC_CK(cudaMemsetAsync(ctx->p2p_start.p, 0, sizeof(int) * ((size_t)ctx->ncell + 1), st));
     k_trav_init<<<1, 1, 0, st>>>(ctx->front[0].p, ctx->d_cnt);
     int nsteps = 2 * (maxl + 1) + 2;
     ctx->launches += 1 + nsteps;
     for (int s = 0; s < nsteps; s++)
       k_trav_step<<<148 * 8, 256, 0, st>>>(s, ctx->front[s & 1].p, ctx->front[(s + 1) & 1].p, ctx->fcap, ctx->d_cnt,
                                            cvm, theta2, prm.variant == TC_VARIANT_TOP, sbits, ctx->m2l.p, ctx->mcap,
-                                           ctx->p2p.p, ctx->pcap, ctx->d_err, mac);
+                                           ctx->p2p.p, ctx->pcap, ctx->d_err, ctx->m2l_start.p, ctx->p2p_start.p,
+                                           mac);
     TcTravCounters hc;
     TC_CK(cudaMemcpyAsync(&hc, ctx->d_cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
     TC_CK(cudaMemcpyAsync(&herr, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
@@ -906,28 +926,30 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
     }
     if (attempt == 5) return TC_ERR_CAPACITY;
   }
-  // ---- sort lists and build per-target offsets
-  int kbits = 2 * sbits;
+  // ---- per-target offsets and sources in order
   {
     size_t nm = ctx->n_m2l, np = ctx->n_p2p;
-    size_t mx = nm > np ? nm : np;
-    if (mx < (size_t)n) mx = (size_t)n;
-    size_t hist_need = 257 * ((mx + kRsTile - 1) / kRsTile + 1) + 1024;
-    TC_CK(ctx->hist.ensure(hist_need));
-    TC_CK(ctx->m2l_alt.ensure(nm + 1));
-    TC_CK(ctx->p2p_alt.ensure(np + 1));
-    ctx->launches += radix_sort(ctx->m2l.p, nullptr, ctx->m2l_alt.p, nullptr, (int)nm, kbits, ctx->hist.p, st);
-    ctx->launches += radix_sort(ctx->p2p.p, nullptr, ctx->p2p_alt.p, nullptr, (int)np, kbits, ctx->hist.p, st);
-    ctx->launches += 5;
-    TC_CK(ctx->m2l_start.ensure(ctx->ncell + 1));
-    TC_CK(ctx->p2p_start.ensure(ctx->ncell + 1));
     TC_CK(ctx->m2l_src.ensure(nm + 1));
     TC_CK(ctx->p2p_src.ensure(np + 1));
     TC_CK(ctx->m2l_tl.ensure(ctx->ncell));
     TC_CK(ctx->p2p_tl.ensure(ctx->ncell));
     TC_CK(ctx->leaves.ensure(ctx->ncell));
-    k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->m2l.p, nm, ctx->ncell, sbits, ctx->m2l_start.p, ctx->m2l_src.p);
-    k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->p2p.p, np, ctx->ncell, sbits, ctx->p2p_start.p, ctx->p2p_src.p);
+    if (ctx->ncell <= kListMaxCells) {
+      TC_CK(ctx->hist.ensure((size_t)ctx->ncell / 4096 + 64));
+      list_build(ctx, ctx->m2l.p, nm, ctx->ncell, ctx->ncell, sbits, ctx->m2l_start.p, ctx->m2l_src.p, nullptr, nullptr);
+      list_build(ctx, ctx->p2p.p, np, ctx->ncell, ctx->ncell, sbits, ctx->p2p_start.p, ctx->p2p_src.p, nullptr, nullptr);
+    } else {
+      const size_t mx = std::max(std::max(nm, np), (size_t)n);
+      TC_CK(ctx->hist.ensure(257 * ((mx + kRsTile - 1) / kRsTile + 1) + 1024));
+      TC_CK(ctx->m2l_alt.ensure(nm + 1));
+      TC_CK(ctx->p2p_alt.ensure(np + 1));
+      ctx->launches += radix_sort(ctx->m2l.p, nullptr, ctx->m2l_alt.p, nullptr, (int)nm, 2 * sbits, ctx->hist.p, st);
+      ctx->launches += radix_sort(ctx->p2p.p, nullptr, ctx->p2p_alt.p, nullptr, (int)np, 2 * sbits, ctx->hist.p, st);
+      k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->m2l.p, nm, ctx->ncell, sbits, ctx->m2l_start.p, ctx->m2l_src.p);
+      k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->p2p.p, np, ctx->ncell, sbits, ctx->p2p_start.p, ctx->p2p_src.p);
+      ctx->launches += 2;
+    }
+    ctx->launches += 3;
     TC_CK(cudaMemsetAsync(ctx->d_small, 0, 4 * sizeof(unsigned), st));
     k_list_targets<<<nblocks(ctx->ncell, 256), 256, 0, st>>>(ctx->m2l_start.p, ctx->ncell, ctx->m2l_tl.p, ctx->d_small);
     k_list_targets<<<nblocks(ctx->ncell, 256), 256, 0, st>>>(ctx->p2p_start.p, ctx->ncell, ctx->p2p_tl.p, ctx->d_small + 1);
@@ -1157,6 +1179,8 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
   // ---- traversal
   const int sbits = ctx->gsbits;
   const double theta2 = prm.theta * prm.theta;
+  cudaMemsetAsync(ctx->m2l_start.p, 0, sizeof(int) * ((size_t)ccap + 1), st);
+  cudaMemsetAsync(ctx->p2p_start.p, 0, sizeof(int) * ((size_t)ccap + 1), st);
   k_trav_init<<<1, 1, 0, st>>>(ctx->front[0].p, ctx->d_cnt);
   const int nsteps = 2 * (TC_MAX_LEVEL + 1) + 2;
   {
@@ -1165,27 +1189,24 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
     for (int s = 0; s < nsteps; s++)
       k_trav_step<<<148 * 8, 256, 0, st>>>(s, ctx->front[s & 1].p, ctx->front[(s + 1) & 1].p, ctx->fcap, ctx->d_cnt,
                                            cv, theta2, prm.variant == TC_VARIANT_TOP, sbits, ctx->m2l.p, ctx->mcap,
-                                           ctx->p2p.p, ctx->pcap, ctx->d_err, mac);
+                                           ctx->p2p.p, ctx->pcap, ctx->d_err, ctx->m2l_start.p, ctx->p2p_start.p,
+                                           mac);
   }
   L += 1 + nsteps;
   graph_check(ctx, "traversal");
-  // ---- sort lists (counts on the device) and per-target offsets
-  const int kbits = 2 * sbits;
-  unsigned long long *km = nullptr, *kp = nullptr;
-  L += radix_sort(ctx->m2l.p, nullptr, ctx->m2l_alt.p, nullptr, (int)ctx->mcap, kbits, ctx->hist.p, st, 0,
-                  &ctx->d_cnt->n_m2l, &km);
-  L += radix_sort(ctx->p2p.p, nullptr, ctx->p2p_alt.p, nullptr, (int)ctx->pcap, kbits, ctx->hist.p, st, 0,
-                  &ctx->d_cnt->n_p2p, &kp);
-  k_list_csr<<<148 * 8, 256, 0, st>>>(km, ctx->mcap, ccap, sbits, ctx->m2l_start.p, ctx->m2l_src.p,
-                                      &ctx->d_cnt->n_m2l, d_ncell);
-  k_list_csr<<<148 * 8, 256, 0, st>>>(kp, ctx->pcap, ccap, sbits, ctx->p2p_start.p, ctx->p2p_src.p,
-                                      &ctx->d_cnt->n_p2p, d_ncell);
+  // ---- per-target offsets and sources in order (counts on the device)
+  const long long before_lists = ctx->launches;
+  list_build(ctx, ctx->m2l.p, ctx->mcap, ccap, ctx->glist_cells, sbits, ctx->m2l_start.p, ctx->m2l_src.p,
+             &ctx->d_cnt->n_m2l, d_ncell);
+  list_build(ctx, ctx->p2p.p, ctx->pcap, ccap, ctx->glist_cells, sbits, ctx->p2p_start.p, ctx->p2p_src.p,
+             &ctx->d_cnt->n_p2p, d_ncell);
+  L += ctx->launches - before_lists;
   cudaMemsetAsync(ctx->d_small, 0, 4 * sizeof(unsigned), st);
   k_list_targets<<<nblocks(ccap, 256), 256, 0, st>>>(ctx->m2l_start.p, ccap, ctx->m2l_tl.p, ctx->d_small, d_ncell);
   k_list_targets<<<nblocks(ccap, 256), 256, 0, st>>>(ctx->p2p_start.p, ccap, ctx->p2p_tl.p, ctx->d_small + 1,
                                                      d_ncell);
   k_leaf_list<<<nblocks(ccap, 256), 256, 0, st>>>(ccap, cv.nchild, ctx->leaves.p, ctx->d_small + 2, d_ncell);
-  L += 5;
+  L += 3;
   graph_check(ctx, "list sort and offsets");
   graph_event(ctx, 3, st);
   // ---- far field and near field
@@ -1569,6 +1590,7 @@ tc_status tc_create(const tc_params* prm, tc_ctx** out) {
     return TC_ERR_CUDA;
   }
   set_attrs(prm->p);
+  cudaFuncSetAttribute(k_list_order, cudaFuncAttributeMaxDynamicSharedMemorySize, kListMaxCells / 8 + 64);
   *out = ctx;
   return TC_OK;
 }
@@ -2046,9 +2068,8 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
   ctx->mcap = ctx->m2l.n;
   ctx->pcap = ctx->p2p.n;
   ctx->fcap = std::min(ctx->front[0].n, ctx->front[1].n);
-  size_t mx = std::max(std::max(ctx->mcap, ctx->pcap), N);
-  if (ctx->m2l_alt.ensure(ctx->mcap + 1) || ctx->p2p_alt.ensure(ctx->pcap + 1) ||
-      ctx->hist.ensure(257 * ((mx + kRsTile - 1) / kRsTile + 1) + 1024) || ctx->m2l_start.ensure(ccap + 1) ||
+  if (ctx->hist.ensure(std::max(257 * ((N + kRsTile - 1) / kRsTile + 1) + 1024, ccap / 4096 + 64)) ||
+      ctx->m2l_start.ensure(ccap + 1) ||
       ctx->p2p_start.ensure(ccap + 1) || ctx->m2l_src.ensure(ctx->mcap + 1) || ctx->p2p_src.ensure(ctx->pcap + 1) ||
       ctx->m2l_tl.ensure(ccap) || ctx->p2p_tl.ensure(ccap) || ctx->leaves.ensure(ccap) ||
       ctx->expn.ensure(ccap * NT * (jerk ? 4 : 2)) || ctx->bpart.ensure(6 * 148 * 4) ||
@@ -2062,8 +2083,12 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
     return;
   // orders are selected in the graph once an evaluation of these bodies left its |a| behind
   ctx->gselect = ctx->prm.selector > 0 && ctx->amag_n == n;
+  // the list keys and bitmaps cover 25 % more cells than this tree has (more overflow a replay, as ccap
+  // would), as far as the bitmap goes
+  ctx->glist_cells = (int)std::min(std::min(ccap, (size_t)(ctx->ncell * 1.25) + 1024), (size_t)kListMaxCells);
+  if (ctx->ncell > ctx->glist_cells) return;
   int sb = 1;
-  while (((size_t)1 << sb) < ccap) sb++;
+  while (((size_t)1 << sb) < (size_t)ctx->glist_cells) sb++;
   ctx->gsbits = sb;
   // judge targets (the same seeded bodies as the normal path's judge)
   ctx->gjudge_nt = 0;

@@ -121,13 +121,19 @@ __global__ void k_pair_features(int K, const int* __restrict__ pt, const int* __
   for (int i = 0; i < TC_NFEAT; i++) feat[(size_t)k * TC_NFEAT + i] = f[i];
 }
 
-__global__ void k_gather_pairs(int K, const unsigned long long* __restrict__ keys, const long long* __restrict__ idx,
-                               int sbits, int* __restrict__ pt, int* __restrict__ ps) {
+// pairs idx[k] of the per-target source lists (ncell targets), counted through the lists in order
+__global__ void k_gather_pairs(int K, int ncell, const int* __restrict__ start, const int* __restrict__ src,
+                               const long long* __restrict__ idx, int* __restrict__ pt, int* __restrict__ ps) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= K) return;
-  unsigned long long key = keys[idx[k]];
-  pt[k] = (int)(key >> sbits);
-  ps[k] = (int)(key & ((1ull << sbits) - 1ull));
+  const int at = (int)idx[k];
+  int lo = 0, hi = ncell;  // the last target with start <= at
+  while (lo + 1 < hi) {
+    const int mid = (lo + hi) / 2;
+    if (start[mid] <= at) lo = mid; else hi = mid;
+  }
+  pt[k] = lo;
+  ps[k] = src[at];
 }
 
 }  // namespace tc
