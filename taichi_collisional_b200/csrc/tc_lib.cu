@@ -461,6 +461,37 @@ static TcP2PWork p2p_plan(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigne
   return W;
 }
 
+// the octree of the Morton-sorted bodies, level by level
+static void tree_levels(tc_ctx* ctx, int n, TcBodies b, TcCells cv) {
+  cudaStream_t st = ctx->stream;
+  if (n <= kTreeSmallN) {
+    k_tree_small<<<1, kTreeSmallThreads, 0, st>>>(n, ctx->prm.ncrit, b, cv, ctx->d_lv, ctx->split_off.p, ctx->d_root,
+                                                  (int)ctx->ccap, ctx->d_err);
+    ctx->launches++;
+    return;
+  }
+  k_tree_root<<<1, 1, 0, st>>>(n, cv, ctx->d_root, ctx->d_lv);
+  ctx->launches += 1 + 3 * (TC_MAX_LEVEL + 1);
+  const int tgrid = 148 * 8;
+  for (int l = 0; l < TC_MAX_LEVEL + 1; l++) {
+    k_tree_split<<<tgrid, 128, 0, st>>>(l, ctx->prm.ncrit, b, cv, ctx->d_lv, ctx->split_off.p, ctx->d_err);
+    k_tree_scan<<<1, 1024, 0, st>>>(l, cv, ctx->d_lv, (int)ctx->ccap, ctx->d_err);
+    k_tree_emit<<<tgrid, 128, 0, st>>>(l, cv, ctx->d_lv, ctx->split_off.p, ctx->d_root);
+  }
+}
+
+// the Morton keys and indices in key order (ending in keys / vals)
+static void sort_bodies(tc_ctx* ctx, int n) {
+  if (n <= kTreeSmallN) {
+    k_sort_small<<<1, kTreeSmallThreads, 0, ctx->stream>>>(n, ctx->keys.p, ctx->vals.p, ctx->keys_alt.p,
+                                                           ctx->vals_alt.p);
+    ctx->launches++;
+  } else {
+    ctx->launches += radix_sort(ctx->keys.p, ctx->vals.p, ctx->keys_alt.p, ctx->vals_alt.p, n, 63, ctx->hist.p,
+                                ctx->stream);
+  }
+}
+
 // per-target offsets and ordered sources of one list from the traversal's counts (in tgt_start) and keys;
 // hist: scan scratch.  bits: cells the bitmap covers
 static void list_build(tc_ctx* ctx, const unsigned long long* keys, size_t n, int ncell, int bits, int sbits,
@@ -587,7 +618,7 @@ static cudaError_t select_orders(tc_ctx* ctx, TcCells cv, int n, int ntl, const 
 }
 
 // whether the FP64 M2L gives every target a warp (tc_m2l_warp.cuh)
-static bool m2l_by_warp(bool jerk, int n) { return (long long)n * (jerk ? 2 : 1) >= kM2LWarpN; }
+static bool m2l_by_warp(int n) { return n >= kM2LWarpN; }
 
 // the FP64 M2L of order Q over the target list: persistent grids (one CTA per SM) taking targets
 // from the counter `next`, with `tend` one order class's range of each list
@@ -596,7 +627,7 @@ static void m2l_launch(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* 
                        const int* src, const int* tend, unsigned* next) {
   cudaStream_t st = ctx->stream;
   const int grid = std::max(1, std::min(ntl, ctx->nsm));
-  const bool by_warp = m2l_by_warp(JERK, n);
+  const bool by_warp = m2l_by_warp(n);
   for (int arr = 0; arr < (JERK && !by_warp ? 2 : 1); arr++) {
     cudaMemsetAsync(next, 0, sizeof(unsigned), st);
     if (by_warp) {
@@ -619,7 +650,7 @@ static void m2l_launch(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* 
 // packed source expansions of the M2L by warps (nc cells; the buffer is reserved in a capture)
 template <int P, bool JERK>
 static cudaError_t m2l_pack(tc_ctx* ctx, TcCells cv, int n, int nc, const int* ncdev) {
-  if (!m2l_by_warp(JERK, n)) return cudaSuccess;
+  if (!m2l_by_warp(n)) return cudaSuccess;
   constexpr int NA = JERK ? 2 : 1;
   cudaError_t e = ctx->mpk.ensure((size_t)nc * NA * tc_pk_off(P + 1));
   if (e != cudaSuccess) return e;
@@ -818,14 +849,7 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
   ctx->ncell = 0;
   // ---- tree levels
   TcCells cv = cells_view(ctx, NT);
-  k_tree_root<<<1, 1, 0, st>>>(n, cv, ctx->d_root, ctx->d_lv);
-  ctx->launches += 1 + 3 * (TC_MAX_LEVEL + 1);
-  int tgrid = 148 * 8;
-  for (int l = 0; l < TC_MAX_LEVEL + 1; l++) {
-    k_tree_split<<<tgrid, 128, 0, st>>>(l, prm.ncrit, b, cv, ctx->d_lv, ctx->split_off.p, ctx->d_err);
-    k_tree_scan<<<1, 1024, 0, st>>>(l, cv, ctx->d_lv, (int)ctx->ccap, ctx->d_err);
-    k_tree_emit<<<tgrid, 128, 0, st>>>(l, cv, ctx->d_lv, ctx->split_off.p, ctx->d_root);
-  }
+  tree_levels(ctx, n, b, cv);
   TC_CK(cudaMemcpyAsync(&ctx->lv, ctx->d_lv, sizeof(TcLevels), cudaMemcpyDeviceToHost, st));
   unsigned herr = 0;
   TC_CK(cudaMemcpyAsync(&herr, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
@@ -1143,14 +1167,9 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
   int* d_count = &ctx->d_lv->count[0];
   long long L = 0;
   // ---- tree levels (as run_fmm)
-  k_tree_root<<<1, 1, 0, st>>>(n, cv, ctx->d_root, ctx->d_lv);
-  const int tgrid = 148 * 8;
-  for (int l = 0; l < TC_MAX_LEVEL + 1; l++) {
-    k_tree_split<<<tgrid, 128, 0, st>>>(l, prm.ncrit, b, cv, ctx->d_lv, ctx->split_off.p, ctx->d_err);
-    k_tree_scan<<<1, 1024, 0, st>>>(l, cv, ctx->d_lv, ccap, ctx->d_err);
-    k_tree_emit<<<tgrid, 128, 0, st>>>(l, cv, ctx->d_lv, ctx->split_off.p, ctx->d_root);
-  }
-  L += 1 + 3 * (TC_MAX_LEVEL + 1);
+  const long long before_tree = ctx->launches;
+  tree_levels(ctx, n, b, cv);
+  L += ctx->launches - before_tree;
   graph_check(ctx, "tree");
   graph_event(ctx, 1, st);
   // ---- expansions (capacity-strided) and upward pass
@@ -1820,7 +1839,8 @@ static tc_status evaluate_impl(tc_ctx* ctx, int n, const double* x, const double
       k_bounds_final<<<1, kBoundsThreads, 0, st>>>(nb, ctx->bpart.p, ctx->d_root, ctx->prm.use_shift, ctx->prm.shift_u[0],
                                       ctx->prm.shift_u[1], ctx->prm.shift_u[2]);
       k_morton<<<nblocks(n, 256), 256, 0, st>>>(n, dx, dy, dz, ctx->d_root, ctx->keys.p, ctx->vals.p);
-      ctx->launches += 4 + radix_sort(ctx->keys.p, ctx->vals.p, ctx->keys_alt.p, ctx->vals_alt.p, n, 63, ctx->hist.p, st);
+      sort_bodies(ctx, n);
+      ctx->launches += 4;
       k_gather_bodies<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->vals.p, dx, dy, dz, dm, dvx, dvy, dvz, df, b);
       run_fn f = pick(ctx->prm.p, jerk);
       if (!f) return TC_ERR_UNSUPPORTED;
@@ -1988,7 +2008,9 @@ static void graph_issue(tc_ctx* ctx, int n, const double* const* in, const unsig
   k_bounds_final<<<1, kBoundsThreads, 0, st>>>(nb, ctx->bpart.p, ctx->d_root, ctx->prm.use_shift, ctx->prm.shift_u[0],
                                   ctx->prm.shift_u[1], ctx->prm.shift_u[2]);
   k_morton<<<nblocks(n, 256), 256, 0, st>>>(n, dx, dy, dz, ctx->d_root, ctx->keys.p, ctx->vals.p);
-  L += 4 + radix_sort(ctx->keys.p, ctx->vals.p, ctx->keys_alt.p, ctx->vals_alt.p, n, 63, ctx->hist.p, st);
+  const long long before_sort = ctx->launches;
+  sort_bodies(ctx, n);
+  L += 4 + ctx->launches - before_sort;
   k_gather_bodies<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->vals.p, dx, dy, dz, dm, dvx, dvy, dvz, df, b);
   graph_check(ctx, "inputs and Morton sort");
   f(ctx, n);
@@ -2074,7 +2096,7 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
       ctx->m2l_tl.ensure(ccap) || ctx->p2p_tl.ensure(ccap) || ctx->leaves.ensure(ccap) ||
       ctx->expn.ensure(ccap * NT * (jerk ? 4 : 2)) || ctx->bpart.ensure(6 * 148 * 4) ||
       p2p_reserve(ctx, n, ccap, jerk ? 7 : 4) ||
-      (m2l_by_warp(jerk, n) && ctx->mpk.ensure(ccap * (jerk ? 2 : 1) * tc_pk_off(ctx->prm.p + 1))))
+      (m2l_by_warp(n) && ctx->mpk.ensure(ccap * (jerk ? 2 : 1) * tc_pk_off(ctx->prm.p + 1))))
     return;
   if (ctx->prm.selector > 0 &&
       (ctx->cell_pn.ensure(ccap * (ctx->prm.p + 1)) || ctx->cell_scale.ensure(ccap) || ctx->body_scale.ensure(N) ||

@@ -31,10 +31,10 @@
 
 namespace tc {
 
-// below this many bodies times expansions there are too few targets (about one per 15 bodies) for the
-// GPU's warps, and k_m2l's four warps per batch of pairs finish sooner (top tree, p = 8: N = 16,384
-// 0.125 ms against 0.18; N = 131,072 1.48 against 1.27)
-constexpr int kM2LWarpN = 65536;
+// below this many bodies there are too few targets (about one per 15 bodies) to keep the GPU's warps even,
+// and k_m2l's four warps per batch of pairs finish sooner (jerks, p = 10: N = 65,537 2.6 ms against 3.0,
+// N = 131,072 4.3 against 3.7; top tree, p = 8: N = 16,384 0.125 against 0.18, N = 131,072 1.48 against 1.27)
+constexpr int kM2LWarpN = 98304;
 
 // ---- packed source expansions: degree d at tc_pk_off(d), (2 d + 1) rounded up to 4 doubles
 __host__ __device__ constexpr int tc_pk_width(int d) { return (2 * d + 1 + 3) / 4 * 4; }

@@ -160,8 +160,18 @@ __global__ void k_trav_step(int s, const int2* __restrict__ fin, int2* __restric
     }
     // a pair's key: its rank among its target's pairs so far, target, source
     unsigned long long key = ((unsigned long long)(unsigned)i << sbits) | (unsigned)j;
-    if (act == 0 || act == 1)
-      key |= (unsigned long long)atomicAdd(act == 0 ? m2l_cnt + i : p2p_cnt + i, 1) << (2 * sbits);
+    {
+      // one atomic for all lanes of the warp with the same target and list (neighbours in the frontier
+      // are children of one pair)
+      const bool emit = act == 0 || act == 1;
+      const unsigned lane = threadIdx.x & 31;
+      const unsigned peers = __match_any_sync(0xffffffffu, emit ? 2u * (unsigned)i + (unsigned)act : 0xffffffffu);
+      const int lead = __ffs(peers) - 1;
+      int rank = 0;
+      if (emit && (int)lane == lead) rank = atomicAdd(act == 0 ? m2l_cnt + i : p2p_cnt + i, __popc(peers));
+      rank = __shfl_sync(0xffffffffu, rank, lead) + __popc(peers & ((1u << lane) - 1u));
+      if (emit) key |= (unsigned long long)rank << (2 * sbits);
+    }
     unsigned long long o = tc_warp_append(&cnt->n_m2l, act == 0);
     if (act == 0) {
       if (o < m2l_cap) m2l[o] = key; else tc_set_err(err, TC_EBIT_M2L_CAP);

@@ -324,40 +324,43 @@ __global__ void k_tree_root(int n, TcCells c, const TcRootInfo* root, TcLevels* 
   lv->start[0] = 0; lv->count[0] = 1; lv->start[1] = 1; lv->ncell = 1;
 }
 
-// decide splits of the cells of level l; off[8*k + o] = first body of octant o
+// first body of octant q in the sorted bodies [beg, end) of a cell centred at (X, Y, Z): by counting up to
+// 32 bodies, else by binary search
+__device__ __forceinline__ int tc_octant_begin(const TcBodies& b, int beg, int end, int q, double X, double Y,
+                                               double Z) {
+  if (q == 0) return beg;
+  if (end - beg <= 32) {
+    int n = 0;
+    for (int i = beg; i < end; i++) n += tc_octant(b.x[i], b.y[i], b.z[i], X, Y, Z) < q;
+    return beg + n;
+  }
+  int left = beg, right = end;
+  while (left < right - 1) {
+    int mid = (left + right) / 2;
+    if (tc_octant(b.x[mid], b.y[mid], b.z[mid], X, Y, Z) >= q) right = mid; else left = mid;
+  }
+  return left + 1;
+}
+
+// decide splits of the cells of level l; off[8*k + o] = first body of octant o.  Eight lanes per cell, one
+// per octant (a thread that searches the octants in turn is seven chains of dependent loads long).
 __global__ void k_tree_split(int l, int ncrit, const TcBodies b, TcCells c, const TcLevels* lv, int* __restrict__ off,
                              unsigned int* err) {
-  int cnt = lv->count[l], st = lv->start[l];
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
-    int ci = st + k;
-    int beg = c.begin[ci], nb = c.nbody[ci], end = beg + nb;
-    double X = c.gx[ci], Y = c.gy[ci], Z = c.gz[ci];
-    if (nb <= ncrit) { c.nchild[ci] = 0; continue; }
-    if (l >= TC_MAX_LEVEL) { c.nchild[ci] = 0; tc_set_err(err, TC_EBIT_DEPTH); continue; }
-    int o8[9];
-    if (nb <= 32) {
-      int size[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int i = beg; i < end; i++) size[tc_octant(b.x[i], b.y[i], b.z[i], X, Y, Z)]++;
-      int o = beg;
-      for (int q = 0; q < 8; q++) { o8[q] = o; o += size[q]; }
-    } else {
-      o8[0] = beg;
-      for (int q = 1; q < 8; q++) {
-        int left = beg, right = end;
-        while (left < right - 1) {
-          int mid = (left + right) / 2;
-          if (tc_octant(b.x[mid], b.y[mid], b.z[mid], X, Y, Z) >= q) right = mid; else left = mid;
-        }
-        o8[q] = left + 1;
-      }
+  const int cnt = lv->count[l], st = lv->start[l];
+  const int q = threadIdx.x & 7, nround = (cnt + 3) & ~3;  // whole warps
+  for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; k < nround; k += (gridDim.x * blockDim.x) >> 3) {
+    const int ci = st + (k < cnt ? k : 0);
+    const int beg = c.begin[ci], nb = c.nbody[ci], end = beg + nb;
+    const bool split = k < cnt && nb > ncrit && l < TC_MAX_LEVEL;
+    const int o = split ? tc_octant_begin(b, beg, end, q, c.gx[ci], c.gy[ci], c.gz[ci]) : beg;
+    const int nx = __shfl_down_sync(0xffffffffu, o, 1, 8), o1 = q == 7 ? end : nx;
+    const unsigned m = __ballot_sync(0xffffffffu, split && o1 > o) >> (threadIdx.x & 24);
+    if (k >= cnt) continue;
+    if (split) off[8 * k + q] = o;
+    if (q == 0) {
+      c.nchild[ci] = split ? __popc(m & 255u) : 0;
+      if (nb > ncrit && l >= TC_MAX_LEVEL) tc_set_err(err, TC_EBIT_DEPTH);
     }
-    o8[8] = end;
-    int nch = 0;
-    for (int q = 0; q < 8; q++) {
-      off[8 * k + q] = o8[q];
-      nch += (q < 7 ? o8[q + 1] : end) - o8[q] > 0;
-    }
-    c.nchild[ci] = nch;
   }
 }
 
@@ -427,6 +430,161 @@ __global__ void k_tree_emit(int l, TcCells c, const TcLevels* lv, const int* __r
       c.gz[ch] = __dadd_rn(c.gz[ci], (q & 4) ? r : -r);
       ch++;
     }
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// Small systems: the key sort and the levels as one CTA each.  At N = 2,000 the 32 sort launches and the
+// 66 level launches took 0.23 and 0.37 ms, nearly all of it launch and load latency.
+// ---------------------------------------------------------------------------------------
+constexpr int kTreeSmallN = 16384, kTreeSmallThreads = 1024;
+
+// the (key, index) pairs in stable key order (eight 8-bit passes, as radix_sort): each warp keeps a
+// contiguous run of the input and the counts of its own digits
+__global__ void __launch_bounds__(kTreeSmallThreads) k_sort_small(int n, unsigned long long* __restrict__ ka,
+                                                                  int* __restrict__ va,
+                                                                  unsigned long long* __restrict__ kb,
+                                                                  int* __restrict__ vb) {
+  constexpr int NW = kTreeSmallThreads / 32;
+  __shared__ uint32_t cnt[NW][256];
+  __shared__ uint32_t dig[256], wtot[8];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int per = ((n + NW - 1) / NW + 31) & ~31, b0 = min(n, w * per), b1 = min(n, b0 + per);
+  for (int pass = 0; pass < 8; pass++) {
+    const int shift = 8 * pass;
+    for (int i = lane; i < 256; i += 32) cnt[w][i] = 0;
+    __syncwarp();
+    for (int i = b0 + lane; i < b1; i += 32) atomicAdd(&cnt[w][(ka[i] >> shift) & 255u], 1u);
+    __syncthreads();
+    // exclusive offsets in (digit, warp) order
+    if (threadIdx.x < 256) {
+      uint32_t t = 0;
+      for (int q = 0; q < NW; q++) {
+        const uint32_t v = cnt[q][threadIdx.x];
+        cnt[q][threadIdx.x] = t;
+        t += v;
+      }
+      uint32_t incl = t;
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+      }
+      if (lane == 31) wtot[w] = incl;
+      dig[threadIdx.x] = incl - t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      uint32_t add = 0;
+      for (int q = 0; q < w; q++) add += wtot[q];
+      dig[threadIdx.x] += add;
+    }
+    __syncthreads();
+    for (int i0 = b0; i0 < b1; i0 += 32) {
+      const int i = i0 + lane;
+      const bool ok = i < b1;
+      const unsigned long long key = ok ? ka[i] : 0ull;
+      const int v = ok ? va[i] : 0;
+      const int d = ok ? (int)((key >> shift) & 255u) : 256;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      uint32_t at = 0;
+      if (ok) at = dig[d] + cnt[w][d] + __popc(peers & lt);
+      __syncwarp();
+      if (ok) {
+        kb[at] = key;
+        vb[at] = v;
+        if ((peers & lt) == 0) cnt[w][d] += __popc(peers);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    unsigned long long* tk = ka; ka = kb; kb = tk;
+    int* tv = va; va = vb; vb = tv;
+  }
+}
+
+// every level of the tree (k_tree_root, then split, scan and emit per level, with the same results)
+__global__ void __launch_bounds__(kTreeSmallThreads) k_tree_small(int n, int ncrit, const TcBodies b, TcCells c,
+                                                                  TcLevels* lv, int* off, const TcRootInfo* root,
+                                                                  int cell_cap, unsigned int* err) {
+  __shared__ int wsum[kTreeSmallThreads / 32];
+  const int T = kTreeSmallThreads, t = threadIdx.x, w = t >> 5, lane = t & 31, q = t & 7;
+  if (t < TC_MAX_LEVEL + 3) { lv->start[t] = 0; lv->count[t] = 0; }
+  __syncthreads();
+  if (t == 0) {
+    c.begin[0] = 0; c.nbody[0] = n; c.nchild[0] = 0; c.child[0] = -1; c.parent[0] = -1; c.level[0] = 0;
+    c.has_sink[0] = 0;
+    c.gx[0] = root->X0[0]; c.gy[0] = root->X0[1]; c.gz[0] = root->X0[2];
+    lv->start[0] = 0; lv->count[0] = 1; lv->start[1] = 1; lv->ncell = 1;
+  }
+  int st = 0, cnt = 1;
+  for (int l = 0; l <= TC_MAX_LEVEL && cnt > 0; l++) {
+    __syncthreads();
+    const double r = tc_level_radius(root->R0, l + 1);
+    const int next = st + cnt;
+    // pass 1: split points and child counts; pass 2: the children, once their number is known to fit
+    int total = 0;
+    for (int k0 = 0; k0 < cnt; k0 += T / 8) {
+      const int k = k0 + (t >> 3), ci = st + (k < cnt ? k : 0);
+      const int beg = c.begin[ci], nb = c.nbody[ci], end = beg + nb;
+      const bool split = k < cnt && nb > ncrit && l < TC_MAX_LEVEL;
+      const int o = split ? tc_octant_begin(b, beg, end, q, c.gx[ci], c.gy[ci], c.gz[ci]) : beg;
+      const int nx = __shfl_down_sync(0xffffffffu, o, 1, 8), o1 = q == 7 ? end : nx;
+      const unsigned m = (__ballot_sync(0xffffffffu, split && o1 > o) >> (t & 24)) & 255u;
+      if (split) off[8 * k + q] = o;
+      const int nch = split ? __popc(m) : 0;
+      if (k < cnt && q == 0 && nb > ncrit && l >= TC_MAX_LEVEL) tc_set_err(err, TC_EBIT_DEPTH);
+      // exclusive scan of nch over the cells of this round (one value per 8 lanes)
+      int incl = q == 0 ? nch : 0;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+      }
+      if (lane == 31) wsum[w] = incl;
+      __syncthreads();
+      int before = total, all = 0;
+      for (int i = 0; i < T / 32; i++) {
+        if (i < w) before += wsum[i];
+        all += wsum[i];
+      }
+      if (k < cnt && q == 0) {
+        c.nchild[ci] = nch;
+        c.child[ci] = nch ? next + before + incl - nch : -1;
+      }
+      total += all;
+      __syncthreads();
+    }
+    const bool over = next + total > cell_cap;  // the level's cells stay leaves (flagged)
+    for (int k = t; over && k < cnt; k += T) {
+      c.nchild[st + k] = 0;
+      c.child[st + k] = -1;
+    }
+    if (over && t == 0) tc_set_err(err, TC_EBIT_CELL_CAP);
+    if (over) total = 0;
+    for (int k = t >> 3; total > 0 && k < ((cnt + 3) & ~3); k += T / 8) {
+      const int ci = st + (k < cnt ? k : 0);
+      const bool split = k < cnt && c.nchild[ci] > 0;
+      const int end = c.begin[ci] + c.nbody[ci];
+      const int o = split ? off[8 * k + q] : 0;
+      const int nx = __shfl_down_sync(0xffffffffu, o, 1, 8), o1 = q == 7 ? end : nx;
+      const unsigned m = (__ballot_sync(0xffffffffu, split && o1 > o) >> (t & 24)) & 255u;
+      if (!split || o1 <= o) continue;
+      const int ch = c.child[ci] + __popc(m & ((1u << q) - 1u));
+      c.begin[ch] = o; c.nbody[ch] = o1 - o; c.nchild[ch] = 0; c.child[ch] = -1; c.parent[ch] = ci;
+      c.level[ch] = l + 1;
+      c.has_sink[ch] = 0;
+      c.gx[ch] = __dadd_rn(c.gx[ci], (q & 1) ? r : -r);
+      c.gy[ch] = __dadd_rn(c.gy[ci], (q & 2) ? r : -r);
+      c.gz[ch] = __dadd_rn(c.gz[ci], (q & 4) ? r : -r);
+    }
+    if (t == 0) {
+      lv->count[l + 1] = total;
+      lv->start[l + 1] = next;
+      lv->start[l + 2] = next + total;
+      lv->ncell = next + total;
+    }
+    st = next;
+    cnt = total;
   }
 }
 
