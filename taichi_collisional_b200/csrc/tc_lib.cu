@@ -500,7 +500,7 @@ static void list_build(tc_ctx* ctx, const unsigned long long* keys, size_t n, in
   ctx->launches += excl_scan(reinterpret_cast<uint32_t*>(tgt_start), ncell + 1, ctx->hist.p, st);
   k_list_scatter<<<(int)std::min<size_t>(nblocks((long long)n, 256) + 1, 148 * 16), 256, 0, st>>>(
       keys, n, ncell, bits, sbits, tgt_start, src, ctx->d_err, ndev, ncdev);
-  const size_t smem = ((size_t)bits + 31) / 32 * 4;
+  const size_t smem = tc_list_bytes(bits);
   const int resident = std::max(1, std::min(16, (int)(220 * 1024 / (smem + 1024))));
   k_list_order<<<std::min(ncell, 148 * resident), kListThreads, smem, st>>>(ncell, bits, tgt_start, src, ncdev);
   ctx->launches += 2;
@@ -1609,7 +1609,8 @@ tc_status tc_create(const tc_params* prm, tc_ctx** out) {
     return TC_ERR_CUDA;
   }
   set_attrs(prm->p);
-  cudaFuncSetAttribute(k_list_order, cudaFuncAttributeMaxDynamicSharedMemorySize, kListMaxCells / 8 + 64);
+  cudaFuncSetAttribute(k_list_order, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)tc_list_bytes(kListMaxCells));
   *out = ctx;
   return TC_OK;
 }

@@ -215,7 +215,10 @@ __global__ void k_trav_step(int s, const int2* __restrict__ fin, int2* __restric
 // 20 ms; N = 12,345: 0.45 of 1.1 ms, launches of a few microseconds each).
 // (ndev, ncdev optional: counts on the device for device-sized launches; n is then the capacity.)
 // ---------------------------------------------------------------------------------------
-constexpr int kListMaxCells = 1792 << 10;  // 224 KB of bits (the ranks in the keys allow 2^21 cells)
+constexpr int kListMaxCells = 1664 << 10;  // 208 KB of bits (the ranks in the keys allow 2^21 cells)
+// shared memory of k_list_order for `cells` cells: the bits, and two counters per block of 1,024
+__host__ __device__ constexpr int tc_list_blocks(int cells) { return (cells + 1023) >> 10; }
+constexpr size_t tc_list_bytes(int cells) { return (size_t)tc_list_blocks(cells) * (128 + 8); }
 
 // cells: cells that the bitmap of k_list_order covers.  Where a replay's list or tree has outgrown what it
 // was planned for (flagged; the host redoes it), every list is made empty, so that what follows in the
@@ -239,28 +242,24 @@ __global__ void k_list_scatter(const unsigned long long* __restrict__ keys, unsi
 }
 
 constexpr int kListThreads = 128;
-// one CTA per target: its segment of src put in ascending order
+// One CTA per target: its segment of src put in ascending order.  A source's place is the number of set
+// bits below it: the counts of the blocks of 1,024 cells before its own, the words of its block before its
+// own, and the bits of its word (reading out the whole bitmap instead took 5 ms a list at N = 4M).  Lists
+// longer than kListHeld entries a thread read it out.
+constexpr int kListHeld = 8;
 __global__ void __launch_bounds__(kListThreads) k_list_order(int ncell, int cells, const int* __restrict__ tgt_start,
                                                              int* __restrict__ src, const int* ncdev = nullptr) {
-  extern __shared__ uint32_t tc_list_bits[];  // a bit for each of `cells` cells
+  extern __shared__ uint32_t tc_list_bits[];  // a bit for each of `cells` cells, then the block counts and sums
   __shared__ int wsum[kListThreads / 32];
   if (ncdev) ncell = *ncdev;
   if (ncell > cells) return;  // the lists are empty
-  const int words = (ncell + 31) >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int per = (words + kListThreads - 1) / kListThreads;  // consecutive words a thread reads out
+  const int nblk = tc_list_blocks(ncell), words = 32 * nblk, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* cnt = reinterpret_cast<int*>(tc_list_bits + 32 * tc_list_blocks(cells));
+  int* pre = cnt + tc_list_blocks(cells);
   for (int i = threadIdx.x; i < words; i += kListThreads) tc_list_bits[i] = 0u;
-  for (int t = blockIdx.x; t < ncell; t += gridDim.x) {
-    const int b = tgt_start[t], e = tgt_start[t + 1];
-    if (e - b < 2) continue;
-    __syncthreads();  // the bitmap is clear
-    for (int k = b + threadIdx.x; k < e; k += kListThreads) {
-      const int s = src[k];
-      atomicOr(&tc_list_bits[s >> 5], 1u << (s & 31));
-    }
-    __syncthreads();
-    const int w0 = threadIdx.x * per, w1 = min(words, w0 + per);
-    int n = 0;
-    for (int i = w0; i < w1; i++) n += __popc(tc_list_bits[i]);
+  for (int i = threadIdx.x; i < nblk; i += kListThreads) cnt[i] = 0;
+  // exclusive sum over the threads of n (every thread takes part)
+  auto before = [&](int n) {
     int incl = n;
     for (int d = 1; d < 32; d <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, incl, d);
@@ -268,13 +267,67 @@ __global__ void __launch_bounds__(kListThreads) k_list_order(int ncell, int cell
     }
     if (lane == 31) wsum[w] = incl;
     __syncthreads();
-    int at = b + incl - n;
+    int at = incl - n;
     for (int i = 0; i < w; i++) at += wsum[i];
-    for (int i = w0; i < w1; i++) {
-      uint32_t m = tc_list_bits[i];
-      if (!m) continue;
-      tc_list_bits[i] = 0u;
-      for (; m; m &= m - 1) src[at++] = 32 * i + __ffs(m) - 1;
+    return at;
+  };
+  for (int t = blockIdx.x; t < ncell; t += gridDim.x) {
+    const int b = tgt_start[t], e = tgt_start[t + 1];
+    if (e - b < 2) continue;
+    __syncthreads();  // bits and counts are clear, wsum is free
+    if (e - b <= kListHeld * kListThreads) {
+      int v[kListHeld];
+#pragma unroll
+      for (int h = 0; h < kListHeld; h++) {
+        const int k = b + h * kListThreads + threadIdx.x;
+        v[h] = k < e ? src[k] : -1;
+        if (v[h] >= 0) {
+          atomicOr(&tc_list_bits[v[h] >> 5], 1u << (v[h] & 31));
+          atomicAdd(&cnt[v[h] >> 10], 1);
+        }
+      }
+      __syncthreads();
+      const int per = (nblk + kListThreads - 1) / kListThreads, i0 = threadIdx.x * per, i1 = min(nblk, i0 + per);
+      int n = 0;
+      for (int i = i0; i < i1; i++) n += cnt[i];
+      int at = before(n);
+      for (int i = i0; i < i1; i++) {
+        pre[i] = at;
+        at += cnt[i];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int h = 0; h < kListHeld; h++) {
+        if (v[h] < 0) continue;
+        int rank = pre[v[h] >> 10];
+        for (int i = v[h] >> 10 << 5; i < v[h] >> 5; i++) rank += __popc(tc_list_bits[i]);
+        rank += __popc(tc_list_bits[v[h] >> 5] & ((1u << (v[h] & 31)) - 1u));
+        src[b + rank] = v[h];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int h = 0; h < kListHeld; h++)
+        if (v[h] >= 0) {
+          tc_list_bits[v[h] >> 5] = 0u;
+          cnt[v[h] >> 10] = 0;
+        }
+    } else {
+      const int per = words / kListThreads + 1;  // consecutive words a thread reads out
+      for (int k = b + threadIdx.x; k < e; k += kListThreads) {
+        const int s = src[k];
+        atomicOr(&tc_list_bits[s >> 5], 1u << (s & 31));
+      }
+      __syncthreads();
+      const int w0 = min(words, (int)threadIdx.x * per), w1 = min(words, w0 + per);
+      int n = 0;
+      for (int i = w0; i < w1; i++) n += __popc(tc_list_bits[i]);
+      int at = b + before(n);
+      for (int i = w0; i < w1; i++) {
+        uint32_t m = tc_list_bits[i];
+        if (!m) continue;
+        tc_list_bits[i] = 0u;
+        for (; m; m &= m - 1) src[at++] = 32 * i + __ffs(m) - 1;
+      }
     }
   }
 }
