@@ -1320,9 +1320,7 @@ static void set_m2l_attrs() {
   cudaFuncSetAttribute(k_m2l_mixed<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
 }
 
-#ifndef TC_ORDERS
 #define TC_ORDERS(X) X(4) X(6) X(8) X(10) X(12) X(16)
-#endif
 
 static run_fn pick(int p, bool jerk) {
   switch (p) {

