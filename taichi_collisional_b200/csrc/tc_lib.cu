@@ -932,7 +932,7 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
       k_trav_step<<<148 * 8, 256, 0, st>>>(s, ctx->front[s & 1].p, ctx->front[(s + 1) & 1].p, ctx->fcap, ctx->d_cnt,
                                            cvm, theta2, prm.variant == TC_VARIANT_TOP, sbits, ctx->m2l.p, ctx->mcap,
                                            ctx->p2p.p, ctx->pcap, ctx->d_err, ctx->m2l_start.p, ctx->p2p_start.p,
-                                           mac);
+                                           ctx->ncell <= kListMaxCells, mac);
     TcTravCounters hc;
     TC_CK(cudaMemcpyAsync(&hc, ctx->d_cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
     TC_CK(cudaMemcpyAsync(&herr, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
@@ -1209,7 +1209,7 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
       k_trav_step<<<148 * 8, 256, 0, st>>>(s, ctx->front[s & 1].p, ctx->front[(s + 1) & 1].p, ctx->fcap, ctx->d_cnt,
                                            cv, theta2, prm.variant == TC_VARIANT_TOP, sbits, ctx->m2l.p, ctx->mcap,
                                            ctx->p2p.p, ctx->pcap, ctx->d_err, ctx->m2l_start.p, ctx->p2p_start.p,
-                                           mac);
+                                           true, mac);
   }
   L += 1 + nsteps;
   graph_check(ctx, "traversal");

@@ -80,7 +80,8 @@ __global__ void k_trav_step(int s, const int2* __restrict__ fin, int2* __restric
                             TcTravCounters* cnt, const TcCells c, double theta2, int top_variant, int sbits,
                             unsigned long long* __restrict__ m2l, unsigned long long m2l_cap,
                             unsigned long long* __restrict__ p2p, unsigned long long p2p_cap, unsigned int* err,
-                            int* __restrict__ m2l_cnt, int* __restrict__ p2p_cnt, const TcMac mac = TcMac()) {
+                            int* __restrict__ m2l_cnt, int* __restrict__ p2p_cnt, bool ranked,
+                            const TcMac mac = TcMac()) {
   unsigned long long nin = cnt->frontier[s % 3];
   if (nin > fcap) nin = fcap;  // an overflowed step was flagged; never read past the buffer
   if (blockIdx.x == 0 && threadIdx.x == 0) cnt->frontier[(s + 2) % 3] = 0;
@@ -158,9 +159,11 @@ __global__ void k_trav_step(int s, const int2* __restrict__ fin, int2* __restric
         act = 3;
       }
     }
-    // a pair's key: its rank among its target's pairs so far, target, source
+    // a pair's key: its rank among its target's pairs so far, target, source.  Keys that a radix sort orders
+    // (trees of more than kListMaxCells cells) carry no rank: its passes are whole bytes, and the last one
+    // would reach past bit 2 sbits into the rank.
     unsigned long long key = ((unsigned long long)(unsigned)i << sbits) | (unsigned)j;
-    {
+    if (ranked) {
       // one atomic for all lanes of the warp with the same target and list (neighbours in the frontier
       // are children of one pair)
       const bool emit = act == 0 || act == 1;
@@ -338,10 +341,10 @@ __global__ void k_list_csr(const unsigned long long* __restrict__ keys, unsigned
   const unsigned long long smask = (1ull << sbits) - 1ull;
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (unsigned long long)gridDim.x * blockDim.x) {
-    unsigned long long key = keys[k] & ((1ull << (2 * sbits)) - 1ull);
+    unsigned long long key = keys[k];
     int t = (int)(key >> sbits);
     src[k] = (int)(key & smask);
-    int tp = k == 0 ? -1 : (int)((keys[k - 1] >> sbits) & smask);
+    int tp = k == 0 ? -1 : (int)(keys[k - 1] >> sbits);
     for (int q = tp + 1; q <= t; q++) tgt_start[q] = (int)k;
     if (k == n - 1)
       for (int q = t + 1; q <= ncell; q++) tgt_start[q] = (int)n;

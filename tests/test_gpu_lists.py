@@ -1,0 +1,48 @@
+"""Interaction lists of trees with more cells than the list bitmaps cover.
+
+Tolerance: an accepted pair's expansion of order p = 4 at theta = 0.5 is cut at theta^(p + 1), 0.03 of the
+pair's own field; the pairs' errors point every way and the near field has none, so the rms error over a
+body's field stays well under a third of that, 1e-2.  A target that loses pairs is off by about its field."""
+import numpy as np
+import pytest
+
+import taichi_collisional_b200 as tcb
+from taichi_collisional_b200 import ics
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+BITMAP_CELLS = 1664 << 10  # kListMaxCells
+KEYS = ("x", "y", "z", "vx", "vy", "vz", "m")
+
+
+def _many_cells(seed):
+    """A cluster whose tree of single-body leaves has about two million cells (keys of 42 bits)."""
+    return {k: torch.tensor(np.ascontiguousarray(a), device="cuda") for k, a in zip(KEYS, ics.plummer(1250000, seed))}
+
+
+def _gravity(**kw):
+    return tcb.Gravity(p=4, ncrit=1, theta=0.5, variant=tcb.VARIANT_JERKS, direct_below=0, **kw)
+
+
+def _outs(n):
+    return {k: torch.empty(n, dtype=torch.float64, device="cuda") for k in ("ax", "ay", "az", "pot", "jx", "jy", "jz")}
+
+
+def _evaluate(g, d, out=None):
+    return g.evaluate(*(d[k] for k in ("x", "y", "z", "m", "vx", "vy", "vz")), out=out)
+
+
+def test_forces_of_a_tree_beyond_the_list_bitmaps():
+    d = _many_cells(31)
+    idx = np.random.default_rng(31).choice(len(d["x"]), 512, replace=False)
+    g = _gravity()
+    out = _evaluate(g, d)
+    assert BITMAP_CELLS < g.stats()["n_cells"] < 1 << 21
+    ref = g.direct_sums(*(d[k] for k in ("x", "y", "z", "m")), idx)
+    g.close()
+    for keys in (("ax", "ay", "az"), ("pot",)):
+        a = np.stack([out[k].cpu().numpy()[idx] for k in keys])
+        b = np.stack([ref[k] for k in keys])
+        err = np.sqrt(np.mean(np.sum((a - b) ** 2, 0)) / np.mean(np.sum(b ** 2, 0)))
+        assert err < 1e-2, (keys, err)
