@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <mutex>
 #include <random>
 #include <string>
@@ -174,6 +175,7 @@ struct tc_ctx {
   DBuf<uint8_t> kd_flags;
   size_t kd_cap = 0;
   size_t fcap = 0, mcap = 0, pcap = 0;
+  size_t fplanned = 0;  // frontier capacity with the headroom of a planned graph (graph_plan)
   // small device structs
   TcRootInfo* d_root = nullptr;
   TcLevels* d_lv = nullptr;
@@ -209,7 +211,7 @@ struct tc_ctx {
   int gjudge_nt = 0;
   long long glaunches = 0;
   int gsbits = 1;
-  int glist_cells = 0;  // cells the graph's list bitmaps cover
+  int glist_cells = 0;  // cells the graph's list bitmaps cover (0: its lists are radix-sorted)
   std::string gfail;  // why the last capture was abandoned (empty: captured)
   std::vector<const void*> gsig;  // buffers and capacities baked into the captured graph
   double gstep_dt = 0.0;          // the graph being planned holds a leapfrog step of this dt
@@ -505,6 +507,20 @@ static void list_build(tc_ctx* ctx, const unsigned long long* keys, size_t n, in
   k_list_order<<<std::min(ncell, 148 * resident), kListThreads, smem, st>>>(ncell, bits, tgt_start, src, ncdev);
   ctx->launches += 2;
 }
+
+// the same of a tree with more than kListMaxCells cells, whose keys carry no rank: radix-sorted (alt: as
+// many keys; hist: the sort's scratch)
+static void list_sort(tc_ctx* ctx, unsigned long long* keys, unsigned long long* alt, size_t n, int ncell, int sbits,
+                      int* tgt_start, int* src, const unsigned long long* ndev, const int* ncdev) {
+  cudaStream_t st = ctx->stream;
+  unsigned long long* sorted = keys;
+  ctx->launches += 1 + radix_sort(keys, nullptr, alt, nullptr, (int)n, 2 * sbits, ctx->hist.p, st, ndev,
+                                  ndev ? &sorted : nullptr);
+  k_list_csr<<<148 * 8, 256, 0, st>>>(sorted, n, ncell, sbits, tgt_start, src, ndev, ncdev);
+}
+
+// counters of a radix sort's scratch
+static size_t sort_scratch(size_t n) { return 257 * ((n + kRsTile - 1) / kRsTile + 1) + 1024; }
 
 // the near field itself: a persistent grid over the items, then the split rows folded
 template <bool JERK>
@@ -964,14 +980,11 @@ static tc_status run_fmm(tc_ctx* ctx, int n) {
       list_build(ctx, ctx->p2p.p, np, ctx->ncell, ctx->ncell, sbits, ctx->p2p_start.p, ctx->p2p_src.p, nullptr, nullptr);
     } else {
       const size_t mx = std::max(std::max(nm, np), (size_t)n);
-      TC_CK(ctx->hist.ensure(257 * ((mx + kRsTile - 1) / kRsTile + 1) + 1024));
+      TC_CK(ctx->hist.ensure(sort_scratch(mx)));
       TC_CK(ctx->m2l_alt.ensure(nm + 1));
       TC_CK(ctx->p2p_alt.ensure(np + 1));
-      ctx->launches += radix_sort(ctx->m2l.p, nullptr, ctx->m2l_alt.p, nullptr, (int)nm, 2 * sbits, ctx->hist.p, st);
-      ctx->launches += radix_sort(ctx->p2p.p, nullptr, ctx->p2p_alt.p, nullptr, (int)np, 2 * sbits, ctx->hist.p, st);
-      k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->m2l.p, nm, ctx->ncell, sbits, ctx->m2l_start.p, ctx->m2l_src.p);
-      k_list_csr<<<148 * 8, 256, 0, st>>>(ctx->p2p.p, np, ctx->ncell, sbits, ctx->p2p_start.p, ctx->p2p_src.p);
-      ctx->launches += 2;
+      list_sort(ctx, ctx->m2l.p, ctx->m2l_alt.p, nm, ctx->ncell, sbits, ctx->m2l_start.p, ctx->m2l_src.p, nullptr, nullptr);
+      list_sort(ctx, ctx->p2p.p, ctx->p2p_alt.p, np, ctx->ncell, sbits, ctx->p2p_start.p, ctx->p2p_src.p, nullptr, nullptr);
     }
     ctx->launches += 3;
     TC_CK(cudaMemsetAsync(ctx->d_small, 0, 4 * sizeof(unsigned), st));
@@ -1209,16 +1222,23 @@ static void run_fmm_graph(tc_ctx* ctx, int n) {
       k_trav_step<<<148 * 8, 256, 0, st>>>(s, ctx->front[s & 1].p, ctx->front[(s + 1) & 1].p, ctx->fcap, ctx->d_cnt,
                                            cv, theta2, prm.variant == TC_VARIANT_TOP, sbits, ctx->m2l.p, ctx->mcap,
                                            ctx->p2p.p, ctx->pcap, ctx->d_err, ctx->m2l_start.p, ctx->p2p_start.p,
-                                           true, mac);
+                                           ctx->glist_cells > 0, mac);
   }
   L += 1 + nsteps;
   graph_check(ctx, "traversal");
   // ---- per-target offsets and sources in order (counts on the device)
   const long long before_lists = ctx->launches;
-  list_build(ctx, ctx->m2l.p, ctx->mcap, ccap, ctx->glist_cells, sbits, ctx->m2l_start.p, ctx->m2l_src.p,
-             &ctx->d_cnt->n_m2l, d_ncell);
-  list_build(ctx, ctx->p2p.p, ctx->pcap, ccap, ctx->glist_cells, sbits, ctx->p2p_start.p, ctx->p2p_src.p,
-             &ctx->d_cnt->n_p2p, d_ncell);
+  if (ctx->glist_cells) {
+    list_build(ctx, ctx->m2l.p, ctx->mcap, ccap, ctx->glist_cells, sbits, ctx->m2l_start.p, ctx->m2l_src.p,
+               &ctx->d_cnt->n_m2l, d_ncell);
+    list_build(ctx, ctx->p2p.p, ctx->pcap, ccap, ctx->glist_cells, sbits, ctx->p2p_start.p, ctx->p2p_src.p,
+               &ctx->d_cnt->n_p2p, d_ncell);
+  } else {
+    list_sort(ctx, ctx->m2l.p, ctx->m2l_alt.p, ctx->mcap, ccap, sbits, ctx->m2l_start.p, ctx->m2l_src.p,
+              &ctx->d_cnt->n_m2l, d_ncell);
+    list_sort(ctx, ctx->p2p.p, ctx->p2p_alt.p, ctx->pcap, ccap, sbits, ctx->p2p_start.p, ctx->p2p_src.p,
+              &ctx->d_cnt->n_p2p, d_ncell);
+  }
   L += ctx->launches - before_lists;
   cudaMemsetAsync(ctx->d_small, 0, 4 * sizeof(unsigned), st);
   k_list_targets<<<nblocks(ccap, 256), 256, 0, st>>>(ctx->m2l_start.p, ccap, ctx->m2l_tl.p, ctx->d_small, d_ncell);
@@ -1774,7 +1794,7 @@ static tc_status evaluate_impl(tc_ctx* ctx, int n, const double* x, const double
   TC_CK(ctx->bod.ensure(ctx->prm.precision != TC_PREC_FP64 ? 13 * N + 2 : 7 * N));
   TC_CK(ctx->bflags.ensure(N)); TC_CK(ctx->perm.ensure(N));
   TC_CK(ctx->outs.ensure(7 * N));
-  TC_CK(ctx->hist.ensure(257 * ((N + kRsTile - 1) / kRsTile + 1) + 1024));
+  TC_CK(ctx->hist.ensure(sort_scratch(N)));
   TC_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), st));
   int direct_below = ctx->prm.direct_below;
   if (direct_below < 0) direct_below = jerk ? 8000 : ctx->prm.ncrit;
@@ -2084,12 +2104,27 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
   ctx->ccap = ccap;
   size_t mcap = std::max(ctx->mcap, (size_t)(ctx->n_m2l * 1.25) + 4096);
   size_t pcap = std::max(ctx->pcap, (size_t)(ctx->n_p2p * 1.25) + 4096);
-  size_t fcap = (size_t)(ctx->fcap * 1.25) + 4096;
+  // (the frontier's once: planning again, for other buffers say, asks for no more)
+  const size_t fcap = ctx->fcap == ctx->fplanned ? ctx->fcap : (size_t)(ctx->fcap * 1.25) + 4096;
   if (ctx->m2l.ensure(mcap) || ctx->p2p.ensure(pcap) || ctx->front[0].ensure(fcap) || ctx->front[1].ensure(fcap)) return;
   ctx->mcap = ctx->m2l.n;
   ctx->pcap = ctx->p2p.n;
-  ctx->fcap = std::min(ctx->front[0].n, ctx->front[1].n);
-  if (ctx->hist.ensure(std::max(257 * ((N + kRsTile - 1) / kRsTile + 1) + 1024, ccap / 4096 + 64)) ||
+  ctx->fcap = ctx->fplanned = std::min(ctx->front[0].n, ctx->front[1].n);
+  // the list keys and bitmaps cover 25 % more cells than this tree has (more overflow a replay, as ccap
+  // would), as far as the bitmap goes; the lists of a larger tree are radix-sorted
+  ctx->glist_cells = 0;
+  if (ctx->ncell <= kListMaxCells)
+    ctx->glist_cells = (int)std::min(std::min(ccap, (size_t)(ctx->ncell * 1.25) + 1024), (size_t)kListMaxCells);
+  if (!ctx->glist_cells && std::max(ctx->mcap, ctx->pcap) > (size_t)INT_MAX - kRsTile) {
+    ctx->gfail = "interaction lists too long for a captured sort";
+    return;
+  }
+  const size_t list_scratch = ctx->glist_cells ? ccap / 4096 + 64 : sort_scratch(std::max(ctx->mcap, ctx->pcap));
+  if (!ctx->glist_cells && (ctx->m2l_alt.ensure(ctx->mcap + 1) || ctx->p2p_alt.ensure(ctx->pcap + 1))) return;
+  int sb = 1;
+  while (((size_t)1 << sb) < (ctx->glist_cells ? (size_t)ctx->glist_cells : ccap)) sb++;
+  ctx->gsbits = sb;
+  if (ctx->hist.ensure(std::max(sort_scratch(N), list_scratch)) ||
       ctx->m2l_start.ensure(ccap + 1) ||
       ctx->p2p_start.ensure(ccap + 1) || ctx->m2l_src.ensure(ctx->mcap + 1) || ctx->p2p_src.ensure(ctx->pcap + 1) ||
       ctx->m2l_tl.ensure(ccap) || ctx->p2p_tl.ensure(ccap) || ctx->leaves.ensure(ccap) ||
@@ -2104,13 +2139,6 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
     return;
   // orders are selected in the graph once an evaluation of these bodies left its |a| behind
   ctx->gselect = ctx->prm.selector > 0 && ctx->amag_n == n;
-  // the list keys and bitmaps cover 25 % more cells than this tree has (more overflow a replay, as ccap
-  // would), as far as the bitmap goes
-  ctx->glist_cells = (int)std::min(std::min(ccap, (size_t)(ctx->ncell * 1.25) + 1024), (size_t)kListMaxCells);
-  if (ctx->ncell > ctx->glist_cells) return;
-  int sb = 1;
-  while (((size_t)1 << sb) < (size_t)ctx->glist_cells) sb++;
-  ctx->gsbits = sb;
   // judge targets (the same seeded bodies as the normal path's judge)
   ctx->gjudge_nt = 0;
   if (ctx->prm.judge_n > 0) {

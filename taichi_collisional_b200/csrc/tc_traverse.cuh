@@ -337,7 +337,10 @@ __global__ void __launch_bounds__(kListThreads) k_list_order(int ncell, int cell
 
 // (target << sbits | source) keys, sorted (trees of more than kListMaxCells cells): per-target offsets
 __global__ void k_list_csr(const unsigned long long* __restrict__ keys, unsigned long long n, int ncell, int sbits,
-                           int* __restrict__ tgt_start, int* __restrict__ src) {
+                           int* __restrict__ tgt_start, int* __restrict__ src,
+                           const unsigned long long* ndev = nullptr, const int* ncdev = nullptr) {
+  if (ndev && *ndev < n) n = *ndev;
+  if (ncdev) ncell = *ncdev;
   const unsigned long long smask = (1ull << sbits) - 1ull;
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (unsigned long long)gridDim.x * blockDim.x) {

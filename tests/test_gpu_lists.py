@@ -1,4 +1,4 @@
-"""Interaction lists of trees with more cells than the list bitmaps cover.
+"""Interaction lists of trees with more cells than the list bitmaps cover, and what planning a graph holds.
 
 Tolerance: an accepted pair's expansion of order p = 4 at theta = 0.5 is cut at theta^(p + 1), 0.03 of the
 pair's own field; the pairs' errors point every way and the near field has none, so the rms error over a
@@ -46,3 +46,43 @@ def test_forces_of_a_tree_beyond_the_list_bitmaps():
         b = np.stack([ref[k] for k in keys])
         err = np.sqrt(np.mean(np.sum((a - b) ** 2, 0)) / np.mean(np.sum(b ** 2, 0)))
         assert err < 1e-2, (keys, err)
+
+
+def test_graph_of_a_tree_beyond_the_list_bitmaps():
+    # captured and replayed like any other; replays take no memory
+    d = _many_cells(32)
+    n = len(d["x"])
+    g, gd = _gravity(), _gravity()
+    g.set_graph(True)
+    out, ref = _outs(n), _outs(n)
+    for step in range(3):
+        for k in "xyz":
+            d[k] += 1e-4 * step * d["v" + k]
+        _evaluate(g, d, out)
+        assert g.graph_ready(), g.graph_note()
+        _evaluate(gd, d, ref)
+        torch.cuda.synchronize()
+        assert g.stats()["n_cells"] == gd.stats()["n_cells"] > BITMAP_CELLS
+        for k in ref:
+            assert torch.equal(out[k], ref[k]), (k, step)
+        free = torch.cuda.mem_get_info()[0]
+        assert step == 0 or free == last, step
+        last = free
+    g.close()
+    gd.close()
+
+
+def test_planning_again_takes_no_more_memory():
+    # other output buffers: a new plan each call, of the same capacities
+    d = {k: torch.tensor(np.ascontiguousarray(a), device="cuda") for k, a in zip(KEYS, ics.plummer(65536, 33))}
+    g = tcb.Gravity(p=4, ncrit=64, theta=0.5, variant=tcb.VARIANT_JERKS)
+    g.set_graph(True)
+    outs = [_outs(65536) for _ in range(2)]
+    free = []
+    for k in range(10):
+        _evaluate(g, d, outs[k % 2])
+        assert g.graph_ready(), g.graph_note()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    g.close()
+    assert len(set(free[2:])) == 1, free
