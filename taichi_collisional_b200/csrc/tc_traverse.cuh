@@ -196,15 +196,11 @@ __global__ void k_trav_step(int s, const int2* __restrict__ fin, int2* __restric
     if (lane == 31 && total) base = atomicAdd(&cnt->frontier[(s + 1) % 3], (unsigned long long)total);
     base = __shfl_sync(0xffffffffu, base, 31) + (incl - nadd);
     if (nadd) {
-      if (base + nadd > fcap) {
-        tc_set_err(err, TC_EBIT_FRONTIER_CAP);
-      } else if (act == 2) {
-        int c0 = c.child[i];
-        for (int q = 0; q < nadd; q++) fout[base + q] = make_int2(c0 + q, j);
-      } else {
-        int c0 = c.child[j];
-        for (int q = 0; q < nadd; q++) fout[base + q] = make_int2(i, c0 + q);
-      }
+      // what fits is written, so that the next step reads no slot below fcap that was never written
+      if (base + nadd > fcap) tc_set_err(err, TC_EBIT_FRONTIER_CAP);
+      const int nw = base >= fcap ? 0 : (int)min((unsigned long long)nadd, fcap - base);
+      const int c0 = c.child[act == 2 ? i : j];
+      for (int q = 0; q < nw; q++) fout[base + q] = act == 2 ? make_int2(c0 + q, j) : make_int2(i, c0 + q);
     }
   }
 }

@@ -86,3 +86,26 @@ def test_planning_again_takes_no_more_memory():
         free.append(torch.cuda.mem_get_info()[0])
     g.close()
     assert len(set(free[2:])) == 1, free
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_context_grows_with_its_system(graph):
+    # a frontier sized for a small system overflows on a large one; the call grows it and answers as a
+    # context that never saw the small one
+    def run(g, n):
+        d = {k: torch.tensor(np.ascontiguousarray(a), device="cuda") for k, a in zip(KEYS, ics.plummer(n, 34))}
+        out = _evaluate(g, d)
+        torch.cuda.synchronize()
+        return out, g.stats()
+
+    kw = dict(p=4, ncrit=64, theta=0.5, variant=tcb.VARIANT_JERKS, direct_below=0)
+    g, fresh = tcb.Gravity(**kw), tcb.Gravity(**kw)
+    g.set_graph(graph)
+    run(g, 300)
+    out, st = run(g, 600000)
+    ref, sr = run(fresh, 600000)
+    assert (st["n_cells"], st["n_m2l"], st["n_p2p"]) == (sr["n_cells"], sr["n_m2l"], sr["n_p2p"])
+    for k in ref:
+        assert torch.equal(out[k], ref[k]), k
+    g.close()
+    fresh.close()
