@@ -1852,6 +1852,7 @@ static tc_status evaluate_impl(tc_ctx* ctx, int n, const double* x, const double
         TC_CK(ctx->split_off.ensure(8 * want_c));
         ctx->ccap = want_c;
       }
+      if (attempt) TC_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), st));  // the overflow of the last attempt
       int nb = 148 * 4;
       TC_CK(ctx->bpart.ensure(6 * nb));
       k_bounds_partial<<<nb, 256, 0, st>>>(n, dx, dy, dz, dm, ctx->bpart.p, ctx->d_err);

@@ -109,3 +109,22 @@ def test_a_context_grows_with_its_system(graph):
         assert torch.equal(out[k], ref[k]), k
     g.close()
     fresh.close()
+
+
+@pytest.mark.parametrize("variant,ncrit", [(tcb.VARIANT_JERKS, 4), (tcb.VARIANT_JERKS, 8), (tcb.VARIANT_TOP, 8)])
+def test_a_tree_of_more_cells_than_the_first_estimate(variant, ncrit):
+    # Small leaves: more than the n / 4 (or 2 n / ncrit) cells that the buffers first hold.  Sums of at most
+    # n = 9,000 FP64 terms in another order than the oracle's: (n + 10) 2^-53 = 1e-12 of the terms' magnitudes,
+    # of which the field is a tenth; twice that.
+    import oracle
+    n = 9000
+    x, y, z, vx, vy, vz, m = ics.plummer(n, 35)
+    o = oracle.evaluate(x, y, z, m, vx, vy, vz, p=4, theta=0.5, ncrit=ncrit, variant=variant)
+    g = tcb.Gravity(p=4, ncrit=ncrit, theta=0.5, variant=variant, direct_below=0)
+    for _ in range(2):
+        out = g.evaluate(x, y, z, m, vx, vy, vz)
+        assert g.stats()["n_cells"] > 2 * n // min(ncrit, 8) + 1024
+        a, b = (np.stack([q[k] for k in ("ax", "ay", "az")]) for q in (out, o))
+        nb = np.linalg.norm(b, axis=0)
+        assert (np.linalg.norm(a - b, axis=0) / np.maximum(nb, 1e-3 * np.sqrt(np.mean(nb ** 2)))).max() < 2e-11
+    g.close()
