@@ -214,7 +214,12 @@ __global__ void k_trav_step(int s, const int2* __restrict__ fin, int2* __restric
 // 20 ms; N = 12,345: 0.45 of 1.1 ms, launches of a few microseconds each).
 // (ndev, ncdev optional: counts on the device for device-sized launches; n is then the capacity.)
 // ---------------------------------------------------------------------------------------
-constexpr int kListMaxCells = 1664 << 10;  // 208 KB of bits (the ranks in the keys allow 2^21 cells)
+// Larger trees are radix-sorted.  A CTA of k_list_order holds a bit per cell, so their CTAs get few (16 an SM
+// up to 96,000 cells, 4 at 400,000, one from 840,000 on) while the sort's time follows the pairs alone.
+// Traversal with the lists in order, bitmaps against sort (ms; p = 4, theta = 0.5): 106,000 cells 2.0 / 2.6,
+// 237,000 5.4 / 6.7, 319,000 11.5 / 14.5, 412,000 9.0 / 9.1, 452,000 13.2 / 12.9, 593,000 7.7 / 5.1,
+// 849,000 38.9 / 18.4, 1,481,000 33.7 / 12.7.
+constexpr int kListMaxCells = 416 << 10;
 // shared memory of k_list_order for `cells` cells: the bits, and two counters per block of 1,024
 __host__ __device__ constexpr int tc_list_blocks(int cells) { return (cells + 1023) >> 10; }
 constexpr size_t tc_list_bytes(int cells) { return (size_t)tc_list_blocks(cells) * (128 + 8); }

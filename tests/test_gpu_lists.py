@@ -12,7 +12,7 @@ from taichi_collisional_b200 import ics
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-BITMAP_CELLS = 1664 << 10  # kListMaxCells
+BITMAP_CELLS = 416 << 10  # kListMaxCells
 KEYS = ("x", "y", "z", "vx", "vy", "vz", "m")
 
 
@@ -38,7 +38,7 @@ def test_forces_of_a_tree_beyond_the_list_bitmaps():
     idx = np.random.default_rng(31).choice(len(d["x"]), 512, replace=False)
     g = _gravity()
     out = _evaluate(g, d)
-    assert BITMAP_CELLS < g.stats()["n_cells"] < 1 << 21
+    assert max(BITMAP_CELLS, 1 << 20) < g.stats()["n_cells"] < 1 << 21
     ref = g.direct_sums(*(d[k] for k in ("x", "y", "z", "m")), idx)
     g.close()
     for keys in (("ax", "ay", "az"), ("pot",)):
@@ -128,3 +128,30 @@ def test_a_tree_of_more_cells_than_the_first_estimate(variant, ncrit):
         nb = np.linalg.norm(b, axis=0)
         assert (np.linalg.norm(a - b, axis=0) / np.maximum(nb, 1e-3 * np.sqrt(np.mean(nb ** 2)))).max() < 2e-11
     g.close()
+
+
+def test_a_replay_that_outgrows_the_list_bitmaps():
+    # planned on a tree just below the bitmaps' limit, replayed on one above it: the call is redone, planned
+    # anew with sorted lists, and the next call replays that
+    n = 280000
+    r = np.random.default_rng(36)
+    d = {k: torch.tensor(np.ascontiguousarray(a), device="cuda") for k, a in zip(KEYS, ics.plummer(n, 36))}
+    for k in "xyz":
+        d[k].copy_(torch.tensor(r.uniform(-1.0, 1.0, n), device="cuda"))
+    g, gd = _gravity(), _gravity()
+    g.set_graph(True)
+    out, ref = _outs(n), _outs(n)
+    for step in range(4):
+        if step == 2:  # close pairs: chains of cells down to each
+            for k in "xyz":
+                d[k][:14000] = d[k][14000:28000] + torch.tensor(1e-3 * r.standard_normal(14000), device="cuda")
+        _evaluate(g, d, out)
+        assert g.graph_ready(), g.graph_note()
+        _evaluate(gd, d, ref)
+        torch.cuda.synchronize()
+        cells = g.stats()["n_cells"]
+        assert cells == gd.stats()["n_cells"] and (cells > BITMAP_CELLS) == (step >= 2) and cells > 350000
+        for k in ref:
+            assert torch.equal(out[k], ref[k]), (k, step)
+    g.close()
+    gd.close()
