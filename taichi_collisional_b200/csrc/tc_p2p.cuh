@@ -908,7 +908,9 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_steps(const int* __restr
             gmax = g1 > gmax ? g1 : gmax;
             dtau = dtp * rr * iv * vdotdr2 * (1.0 + mi * (iv * iv) * invr);
             if (!(dtau < 1.0)) dtau = 1.0;
-            const double g2 = v2 * iv * invr * idtp * (1.0 - 0.5 * dtau);
+            // |dv|: infinite where v2 is (inf * 0 would be NaN, which no comparison keeps)
+            const double sv = __double2hiint(v2) == 0x7ff00000 ? v2 : v2 * iv;
+            const double g2 = sv * invr * idtp * (1.0 - 0.5 * dtau);
             gmax = g2 > gmax ? g2 : gmax;
           } else {
             const double vdotdr2 = (dx * du + dy * dv + dz * dw) / r2;
