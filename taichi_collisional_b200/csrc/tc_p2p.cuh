@@ -495,8 +495,11 @@ __device__ __forceinline__ bool tc_rsqrt_in_range(double x) {
   return (unsigned)(__double2hiint(x) - (123 << 20)) < (unsigned)(1800 << 20);
 }
 
+// A velocity whose difference from another such one is finite, so that 0 times it is 0
+__device__ __forceinline__ bool tc_vel_bounded(double v) { return fabs(v) < 0x1p1023; }
+
 // Two staged sources on one target without a branch between them, so their dependent chains overlap
-// (every source of the tile is one and every velocity is finite, see k_p2p).  A pair at r = 0 adds
+// (every source of the tile is one and every velocity is bounded, see k_p2p).  A pair at r = 0 adds
 // zero; an r^2 outside tc_rsqrt_normal's range takes the library's root.
 template <bool JERK>
 __device__ __forceinline__ void tc_p2p_staged2(const TcTile64<JERK>& T, int s0, int s1, double xi, double yi,
@@ -564,7 +567,8 @@ __global__ void __launch_bounds__(kP2PWarps * 32, JERK ? 4 : 5) k_p2p(const int*
       xi = b.x[i]; yi = b.y[i]; zi = b.z[i];
       if (JERK) { vxi = b.vx[i]; vyi = b.vy[i]; vzi = b.vz[i]; }
     }
-    const bool finite_i = !JERK || __all_sync(0xffffffffu, isfinite(vxi) && isfinite(vyi) && isfinite(vzi));
+    const bool bounded_i =
+        !JERK || __all_sync(0xffffffffu, tc_vel_bounded(vxi) && tc_vel_bounded(vyi) && tc_vel_bounded(vzi));
     TcAcc<JERK> a;
     a.zero();
     int q = it.q, off = it.off, left = it.cnt, q0 = q, cjb, cjn, myj;
@@ -575,10 +579,10 @@ __global__ void __launch_bounds__(kP2PWarps * 32, JERK ? 4 : 5) k_p2p(const int*
     while (cnt > 0) {
       __syncwarp();
       sb.put(T, lane);
-      // every source of the tile is one (x is not NaN) and has a finite velocity
-      const bool plain = finite_i && __all_sync(0xffffffffu, isfinite(sb.x) && (!JERK || (isfinite(sb.u) &&
-                                                                                          isfinite(sb.v) &&
-                                                                                          isfinite(sb.w))));
+      // every source of the tile is one (x is not NaN) and has a bounded velocity
+      const bool plain = bounded_i && __all_sync(0xffffffffu, isfinite(sb.x) && (!JERK || (tc_vel_bounded(sb.u) &&
+                                                                                           tc_vel_bounded(sb.v) &&
+                                                                                           tc_vel_bounded(sb.w))));
       __syncwarp();
       const int now = cnt;
       left -= now;
