@@ -633,8 +633,11 @@ static cudaError_t select_orders(tc_ctx* ctx, TcCells cv, int n, int ntl, const 
   return cudaGetLastError();
 }
 
-// whether the FP64 M2L gives every target a warp (tc_m2l_warp.cuh)
-static bool m2l_by_warp(int n) { return n >= kM2LWarpN; }
+// whether the FP64 M2L gives every target a warp (the rule of tc_m2l_warp.cuh)
+static bool m2l_by_warp(const tc_ctx* ctx, int n) {
+  const tc_params& prm = ctx->prm;
+  return tc_m2l_by_warp(n, prm.ncrit, prm.p, prm.variant == TC_VARIANT_JERKS, ctx->emac);
+}
 
 // the FP64 M2L of order Q over the target list: persistent grids (one CTA per SM) taking targets
 // from the counter `next`, with `tend` one order class's range of each list
@@ -643,7 +646,7 @@ static void m2l_launch(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* 
                        const int* src, const int* tend, unsigned* next) {
   cudaStream_t st = ctx->stream;
   const int grid = std::max(1, std::min(ntl, ctx->nsm));
-  const bool by_warp = m2l_by_warp(n);
+  const bool by_warp = m2l_by_warp(ctx, n);
   for (int arr = 0; arr < (JERK && !by_warp ? 2 : 1); arr++) {
     cudaMemsetAsync(next, 0, sizeof(unsigned), st);
     if (by_warp) {
@@ -666,7 +669,7 @@ static void m2l_launch(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigned* 
 // packed source expansions of the M2L by warps (nc cells; the buffer is reserved in a capture)
 template <int P, bool JERK>
 static cudaError_t m2l_pack(tc_ctx* ctx, TcCells cv, int n, int nc, const int* ncdev) {
-  if (!m2l_by_warp(n)) return cudaSuccess;
+  if (!m2l_by_warp(ctx, n)) return cudaSuccess;
   constexpr int NA = JERK ? 2 : 1;
   cudaError_t e = ctx->mpk.ensure((size_t)nc * NA * tc_pk_off(P + 1));
   if (e != cudaSuccess) return e;
@@ -2131,7 +2134,7 @@ static void graph_plan(tc_ctx* ctx, int n, const TcGraphKey& key, const double* 
       ctx->m2l_tl.ensure(ccap) || ctx->p2p_tl.ensure(ccap) || ctx->leaves.ensure(ccap) ||
       ctx->expn.ensure(ccap * NT * (jerk ? 4 : 2)) || ctx->bpart.ensure(6 * 148 * 4) ||
       p2p_reserve(ctx, n, ccap, jerk ? 7 : 4) ||
-      (m2l_by_warp(n) && ctx->mpk.ensure(ccap * (jerk ? 2 : 1) * tc_pk_off(ctx->prm.p + 1))))
+      (m2l_by_warp(ctx, n) && ctx->mpk.ensure(ccap * (jerk ? 2 : 1) * tc_pk_off(ctx->prm.p + 1))))
     return;
   if (ctx->prm.selector > 0 &&
       (ctx->cell_pn.ensure(ccap * (ctx->prm.p + 1)) || ctx->cell_scale.ensure(ccap) || ctx->body_scale.ensure(N) ||

@@ -31,10 +31,31 @@
 
 namespace tc {
 
-// below this many bodies there are too few targets (about one per 15 bodies) to keep the GPU's warps even,
-// and k_m2l's four warps per batch of pairs finish sooner (jerks, p = 10: N = 65,537 2.6 ms against 3.0,
-// N = 131,072 4.3 against 3.7; top tree, p = 8: N = 16,384 0.125 against 0.18, N = 131,072 1.48 against 1.27)
+// When a target gets a warp.  A work item is one expansion of one target, about n / ncrit targets; with few
+// items the warps end unevenly, and k_m2l's four warps per batch of pairs finish sooner, the more so at low
+// orders, where an item is short.  M2L time of this form over that of k_m2l (98,304 to 2M bodies, ncrit 32 to
+// 256):
+//   theta criterion    items      768          1,536        3,072        12,500
+//                      p =  8     1.12 - 1.30  0.86 - 0.95  0.71 - 0.82  0.62 - 0.74
+//                      p = 10     1.04 - 1.18  0.92 - 0.98  0.82 - 0.89  0.73 - 0.83
+//                      p = 12     0.90 - 1.02  0.81 - 0.88  0.69 - 0.75  0.62 - 0.71
+//                      p = 16     0.85         0.79 - 0.80  0.70 - 0.77  0.66 - 0.73   (384: 0.91)
+// The error-controlled criterion gives a few outlying targets lists many times the others', which one warp
+// walks alone; in the top tree that costs more items,
+//                      items      1,536        3,072        4,096        12,500
+//                      p =  8     1.10         1.06 - 1.18  0.85         0.79
+//                      p = 10     1.58         1.02 - 1.24  0.91         0.81
+//                      p = 12     1.21         0.73 - 0.90  0.71         0.67
+// and in the jerks tree this form is no faster at any size measured up to p = 10 (0.94 to 1.39 up to 31,000
+// items) but from p = 12 on (0.62 to 1.08).  Below 98,304 bodies k_m2l stays; there the items would decide
+// alike (65,537 bodies with jerks, ncrit 64: p = 8 0.85, p = 12 0.79; ncrit 256: p = 10 1.37).
 constexpr int kM2LWarpN = 98304;
+inline bool tc_m2l_by_warp(int n, int ncrit, int p, bool jerk, bool emac) {
+  if (n < kM2LWarpN) return false;
+  const long long items = (long long)n * (jerk ? 2 : 1) / ncrit;
+  if (emac) return p >= 12 ? jerk || items >= 3072 : !jerk && items >= 4096;
+  return items >= (p >= 16 ? 384 : p >= 12 ? 768 : 1536);
+}
 
 // ---- packed source expansions: degree d at tc_pk_off(d), (2 d + 1) rounded up to 4 doubles
 __host__ __device__ constexpr int tc_pk_width(int d) { return (2 * d + 1 + 3) / 4 * 4; }
