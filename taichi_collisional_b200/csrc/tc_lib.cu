@@ -2059,7 +2059,7 @@ static void graph_issue(tc_ctx* ctx, int n, const double* const* in, const unsig
   k_scatter_out<<<nblocks(n, 256), 256, 0, st>>>(n, ctx->perm.p, o, opot, oax, oay, oaz, ojx, ojy, ojz);
   L += 1;
   if (ctx->prm.selector > 0) {  // the next replay's per-target error budget
-    k_amag<<<nblocks(n, 256), 256, 0, st>>>(n, oax, oay, oaz, ctx->amag.p);
+    k_amag<<<nblocks(n, 256), 256, 0, st>>>(n, oax, oay, oaz, ctx->amag.p, ctx->d_err, kGraphCapBits);
     L++;
   }
   if (sdt != 0.0) {  // closing kick by the new accelerations (not after a capacity overflow)

@@ -34,9 +34,12 @@ struct TcClassOrders {
   double comb[TC_PMAX_DEV + 1];
 };
 
-// |a| of each body in caller order (the next evaluation's error budget)
+// |a| of each body in caller order (the next evaluation's error budget); with `err`, not where one of `mask`
+// is set (a replay that outgrew its plan: its accelerations are no budget for the evaluation that redoes it)
 __global__ void k_amag(int n, const double* __restrict__ ax, const double* __restrict__ ay,
-                       const double* __restrict__ az, double* __restrict__ amag) {
+                       const double* __restrict__ az, double* __restrict__ amag, const unsigned* err = nullptr,
+                       unsigned mask = 0u) {
+  if (err && (*err & mask)) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) amag[i] = sqrt(ax[i] * ax[i] + ay[i] * ay[i] + az[i] * az[i]);
 }
