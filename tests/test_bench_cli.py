@@ -40,3 +40,15 @@ def test_reference_arm_prints_the_contract_line():
 def test_reference_arm_other_ranks_print_nothing():
     assert _run(["--impl", "reference", "--n", "4096", "--steps", "1", "--warmup", "1"],
                 env={"RANK": "1", "WORLD_SIZE": "2"}) == []
+
+
+def test_reference_arm_says_at_once_that_its_build_is_absent():
+    # without the reference's CPU build a workload that the one-core port cannot finish in the time budget is
+    # not begun: a line with the reason instead of none
+    import oracle
+    import pytest
+    if oracle.ref_available(oracle.VARIANT_JERKS, 12):
+        pytest.skip("the reference's CPU build is here")
+    lines = _run(["--impl", "reference", "--n", "8192", "--steps", "2", "--warmup", "1", "--ref-budget", "1"])
+    assert len(lines) == 1 and set(lines[0]) == {"impl", "unavailable"} and lines[0]["impl"] == "reference"
+    assert "oracle/_ref" in lines[0]["unavailable"]
