@@ -401,16 +401,14 @@ constexpr int tc_m2l_threads() { return 128 * TcM2LGroups<Q>::G; }
 
 // M2L of order Q <= P over a per-target list (or, with `tend`, one order class's range of it);
 // expansions are stored with order P.  Adds into L (zeroed before the first M2L launch of an
-// evaluation).  One CTA per SM (shared
-// memory), which owns the tensor memory it allocates.  One target per CTA, or, with `next`
-// (a counter zeroed before the launch), a persistent grid whose CTAs take targets in turn.
+// evaluation).  A persistent grid of one CTA per SM (shared memory), which owns the tensor memory it
+// allocates; the CTAs take targets in turn from `next`, zeroed before the launch.
 template <int P, int Q>
 __global__ void __launch_bounds__(tc_m2l_threads<Q>(), 1) k_m2l(const int* __restrict__ tlist, int ntl,
                                                                const int* __restrict__ tstart,
                                                                const int* __restrict__ src, TcCells c,
-                                                               const unsigned* ntldev = nullptr,
-                                                               unsigned* next = nullptr,
-                                                               const int* __restrict__ tend = nullptr) {
+                                                               const unsigned* ntldev, unsigned* next,
+                                                               const int* __restrict__ tend) {
   using SM = TcM2LSmem<Q>;
   using TM = TcM2LTmem<Q>;
   constexpr int NTQ = SM::NT, NTP = (P + 1) * (P + 1);
@@ -419,15 +417,11 @@ __global__ void __launch_bounds__(tc_m2l_threads<Q>(), 1) k_m2l(const int* __res
   extern __shared__ double tc_m2l_smem[];
   __shared__ uint32_t s_tmem;
   __shared__ int s_ti;
-  int ti = blockIdx.x;
   if (ntldev) ntl = (int)*ntldev;  // device-sized launch (graph)
-  if (next) {
-    if (threadIdx.x == 0) s_ti = (int)atomicAdd(next, 1u);
-    __syncthreads();
-    ti = s_ti;
-  }
+  if (threadIdx.x == 0) s_ti = (int)atomicAdd(next, 1u);
+  __syncthreads();
+  int ti = s_ti;
   if (ti >= ntl) return;
-  if (!next && !c.has_sink[tlist[ti]]) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = warp >> 2, w = warp & 3, acol = grp * 32 + lane;
   if (warp == 0) {
@@ -482,7 +476,6 @@ __global__ void __launch_bounds__(tc_m2l_threads<Q>(), 1) k_m2l(const int* __res
     }
     tc_bar_cta();
   }
-  if (!next) break;
   if (threadIdx.x == 0) s_ti = (int)atomicAdd(next, 1u);
   tc_bar_cta();
   ti = s_ti;
