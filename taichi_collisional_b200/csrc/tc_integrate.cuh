@@ -177,13 +177,11 @@ struct TcEvolve {
     const cudaStream_t s = ctx->stream;
     tc_status r;
     if (direct) {
-      // the context's own storage (never the library-wide static array of
-      // tc_evaluate_direct_noalloc, which contexts stepping at once would share)
-      const size_t S = ctx->kd_cap;
-      r = (size_t)ns <= S && direct_with_scratch(ns, X(0, off), X(1, off), X(2, off), nullptr, nullptr, nullptr,
-                                                 X(9, off), fl, ax, ay, az, apot, nullptr, nullptr, nullptr, 0, s,
-                                                 ctx->kd_scratch.p, ctx->kd_index.p, ctx->kd_flags.p, S,
-                                                 ctx->prm.softening * ctx->prm.softening) == cudaSuccess
+      TcOut o;  // the context's own arrays, which no input shares memory with
+      o.ax = ax; o.ay = ay; o.az = az; o.pot = apot;
+      o.jx = o.jy = o.jz = nullptr;
+      r = direct_plain(ns, X(0, off), X(1, off), X(2, off), nullptr, nullptr, nullptr, X(9, off), fl,
+                       ctx->prm.softening * ctx->prm.softening, o, false, s) == cudaSuccess
               ? TC_OK
               : TC_ERR_CUDA;
       st.n_direct++;
@@ -433,12 +431,6 @@ static tc_status tc_evolve_run(tc_ctx* ctx, int n, double* x, double* y, double*
   TC_CK(ctx->ev_u.ensure(mn_at + 2));
   TC_CK(ctx->ev_i.ensure(2 * (size_t)n + 2));
   TC_CK(ctx->ev_f.ensure((size_t)n));
-  // systems of at most kDirectMax bodies are kicked by direct sums (kick_cpu)
-  constexpr size_t kDirectMax = 128;
-  TC_CK(ctx->kd_scratch.ensure(14 * kDirectMax));
-  TC_CK(ctx->kd_index.ensure(kDirectMax));
-  TC_CK(ctx->kd_flags.ensure(kDirectMax));
-  ctx->kd_cap = kDirectMax;
   TcEvolve E;
   E.ctx = ctx;
   double* arr[12] = {x, y, z, ex, ey, ez, vx, vy, vz, m, timestep, pot};

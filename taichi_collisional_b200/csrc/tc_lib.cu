@@ -170,10 +170,6 @@ struct tc_ctx {
   DBuf<uint8_t> ev_f;
   DBuf<uint8_t> ds_flags;
   DBuf<int> ds_idx, ds_tgt;
-  DBuf<double> kd_scratch;  // direct kicks of small systems: 14 arrays of kd_cap entries
-  DBuf<int> kd_index;
-  DBuf<uint8_t> kd_flags;
-  size_t kd_cap = 0;
   size_t fcap = 0, mcap = 0, pcap = 0;
   size_t fplanned = 0;  // frontier capacity with the headroom of a planned graph (graph_plan)
   // small device structs
@@ -447,11 +443,11 @@ static TcP2PWork p2p_plan(tc_ctx* ctx, TcCells cv, int n, int ntl, const unsigne
   cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), st);
   cudaMemsetAsync(ctx->d_small + 12, 0, sizeof(unsigned), st);
   unsigned long long *inter = &ctx->d_cnt->frontier[0], *cost = &ctx->d_cnt->frontier[1];
-  const int gw = std::min(nblocks(ntl, 8), 148 * 8), gp = gw;
+  const int gw = std::min(nblocks(ntl, 8), 148 * 8);
   k_p2p_work<<<gw, 256, 0, st>>>(ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, cv, ctx->p2p_s.p, inter, cost,
                                  ntldev);
   const int K = p2p_units(n);
-  k_p2p_plan<<<gp, 256, 0, st>>>(ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, cv, ctx->p2p_s.p, cost, K,
+  k_p2p_plan<<<gw, 256, 0, st>>>(ctx->p2p_tl.p, ntl, ctx->p2p_start.p, ctx->p2p_src.p, cv, ctx->p2p_s.p, cost, K,
                                  2 * K, ctx->p2p_singles.p, ctx->p2p_items.p, ctx->p2p_rows.p, cnt, ntldev);
   TcP2PWork W;
   W.items = ctx->p2p_items.p;
@@ -1470,9 +1466,10 @@ __global__ void k_fma_probe(T* out, int iters) {
 
 // ----------------------------------------------------------------------------------------
 // Scratch of tc_evaluate_direct_noalloc: a fixed static device array instead of cudaMalloc.
-// Layout: 7 body arrays (x y z m vx vy vz) | 7 output arrays, each TC_NOALLOC_MAX_N doubles.
+// Layout: 7 body arrays (x y z m vx vy vz) of TC_NOALLOC_MAX_N doubles each, copies of the inputs for
+// calls whose outputs share memory with them.
 // ----------------------------------------------------------------------------------------
-static __device__ __align__(256) double g_noalloc_scratch[14 * TC_NOALLOC_MAX_N];
+static __device__ __align__(256) double g_noalloc_scratch[7 * TC_NOALLOC_MAX_N];
 static __device__ __align__(256) int g_noalloc_index[TC_NOALLOC_MAX_N];
 static __device__ __align__(256) uint8_t g_noalloc_flags[TC_NOALLOC_MAX_N];
 
@@ -1511,37 +1508,14 @@ static void direct_launch(int n, const double* x, const double* y, const double*
     k_direct<false><<<nblocks(n, kDirT), kDirThreads, 0, st>>>(n, x, y, z, vx, vy, vz, m, flags, eps2, o, err);
 }
 
-// Direct-sum evaluation that allocates nothing.  Where an output shares memory with an input, the
-// inputs are first copied to working storage the caller provides: S entries per array in
-// `scratch` (7 arrays: x y z m vx vy vz), `index` and `flags` (n <= S).  Shared by
-// tc_evaluate_direct_noalloc (the static array) and the block-time-step integrator's direct kicks.
-static cudaError_t direct_with_scratch(int n, const double* x, const double* y, const double* z, const double* vx,
-                                       const double* vy, const double* vz, const double* m,
-                                       const unsigned char* flags, double* ax, double* ay, double* az, double* pot,
-                                       double* jx, double* jy, double* jz, int jerk, cudaStream_t st,
-                                       double* scratch, int* index, uint8_t* fl, size_t S, double eps2 = 0.0) {
-  TcOut o;
-  o.pot = pot; o.ax = ax; o.ay = ay; o.az = az;
-  o.jx = jerk ? jx : nullptr; o.jy = jerk ? jy : nullptr; o.jz = jerk ? jz : nullptr;
-  const double* in[7] = {x, y, z, m, vx, vy, vz};
-  double* outs[7] = {ax, ay, az, pot, o.jx, o.jy, o.jz};
-  if (!outputs_overlap(n, in, jerk ? 7 : 4, flags, outs, 7)) {
-    if (!jerk && n <= kChainN) {
-      k_direct_chain<<<nblocks(n, kChainT), 256, 0, st>>>(n, x, y, z, m, flags, eps2, o);
-      return cudaGetLastError();
-    }
-    direct_launch(n, x, y, z, vx, vy, vz, m, flags, eps2, o, jerk != 0, nullptr, st);
-    return cudaGetLastError();
-  }
-  TcBodies b;
-  b.x = scratch; b.y = scratch + S; b.z = scratch + 2 * S; b.m = scratch + 3 * S;
-  b.vx = jerk ? scratch + 4 * S : nullptr; b.vy = jerk ? scratch + 5 * S : nullptr;
-  b.vz = jerk ? scratch + 6 * S : nullptr;
-  b.flags = fl;
-  b.perm = index;
-  k_identity<<<nblocks(n, 256), 256, 0, st>>>(n, index);
-  k_gather_bodies<<<nblocks(n, 256), 256, 0, st>>>(n, index, x, y, z, m, vx, vy, vz, flags, b);
-  direct_launch(n, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.m, b.flags, eps2, o, jerk != 0, nullptr, st);
+// The direct sums without a context: no allocation, no status.  No output may share memory with an input.
+static cudaError_t direct_plain(int n, const double* x, const double* y, const double* z, const double* vx,
+                                const double* vy, const double* vz, const double* m, const unsigned char* flags,
+                                double eps2, TcOut o, bool jerk, cudaStream_t st) {
+  if (!jerk && n <= kChainN)
+    k_direct_chain<<<nblocks(n, kChainT), 256, 0, st>>>(n, x, y, z, m, flags, eps2, o);
+  else
+    direct_launch(n, x, y, z, vx, vy, vz, m, flags, eps2, o, jerk, nullptr, st);
   return cudaGetLastError();
 }
 
@@ -1657,7 +1631,7 @@ tc_status tc_destroy(tc_ctx* ctx) {
   ctx->p2p_items.release(); ctx->p2p_rows.release(); ctx->p2p_slots.release();
   ctx->ev_d.release(); ctx->ev_u.release(); ctx->ev_i.release(); ctx->ev_f.release();
   ctx->amag.release(); ctx->body_scale.release(); ctx->cell_scale.release(); ctx->m2l_src2.release();
-  ctx->m2l_off.release(); ctx->cls_rng.release(); ctx->cell_feat.release(); ctx->kd_scratch.release(); ctx->kd_index.release(); ctx->kd_flags.release();
+  ctx->m2l_off.release(); ctx->cls_rng.release(); ctx->cell_feat.release();
   ctx->low_f.release();
   if (ctx->d_root) cudaFree(ctx->d_root);
   if (ctx->d_lv) cudaFree(ctx->d_lv);
@@ -2547,10 +2521,24 @@ tc_status tc_evaluate_direct_noalloc(int n, const double* x, const double* y, co
     }
     D = g_noalloc_dev[dev];
   }
-  return direct_with_scratch(n, x, y, z, vx, vy, vz, m, flags, ax, ay, az, pot, jx, jy, jz, jerk,
-                             (cudaStream_t)stream, D.scratch, D.index, D.flags, TC_NOALLOC_MAX_N) == cudaSuccess
-             ? TC_OK
-             : TC_ERR_CUDA;
+  cudaStream_t st = (cudaStream_t)stream;
+  TcOut o;
+  o.pot = pot; o.ax = ax; o.ay = ay; o.az = az;
+  o.jx = jerk ? jx : nullptr; o.jy = jerk ? jy : nullptr; o.jz = jerk ? jz : nullptr;
+  const double* in[7] = {x, y, z, m, vx, vy, vz};
+  double* outs[7] = {ax, ay, az, pot, o.jx, o.jy, o.jz};
+  if (outputs_overlap(n, in, jerk ? 7 : 4, flags, outs, 7)) {  // sums over copies of the inputs
+    const size_t S = TC_NOALLOC_MAX_N;
+    TcBodies b;
+    b.x = D.scratch; b.y = b.x + S; b.z = b.y + S; b.m = b.z + S;
+    b.vx = jerk ? b.m + S : nullptr; b.vy = jerk ? b.m + 2 * S : nullptr; b.vz = jerk ? b.m + 3 * S : nullptr;
+    b.flags = D.flags;
+    b.perm = D.index;
+    k_identity<<<nblocks(n, 256), 256, 0, st>>>(n, D.index);
+    k_gather_bodies<<<nblocks(n, 256), 256, 0, st>>>(n, D.index, x, y, z, m, vx, vy, vz, flags, b);
+    x = b.x; y = b.y; z = b.z; vx = b.vx; vy = b.vy; vz = b.vz; m = b.m; flags = b.flags;
+  }
+  return direct_plain(n, x, y, z, vx, vy, vz, m, flags, 0.0, o, jerk != 0, st) == cudaSuccess ? TC_OK : TC_ERR_CUDA;
 }
 
 tc_status tc_train_selector(tc_ctx* ctx, int n, const double* x, const double* y, const double* z, const double* vx,
