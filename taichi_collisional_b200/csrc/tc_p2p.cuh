@@ -904,7 +904,11 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_steps(const int* __restr
           if (POS) {
             invr = rsqrt(r2);
             invr2 = invr * invr;
-            const double rr = r2 * invr, iv = rsqrt(v2), rm = rr * mi, qm = rsqrt(rm);
+            // 1 / |dv|, at least 2^-520: where v2 overflowed, |dv| = v2 iv is then infinite and not inf * 0 = NaN,
+            // which no comparison keeps (a finite v2 has a root of 2^-512 or more)
+            double iv = rsqrt(v2);
+            iv = __hiloint2double(max(__double2hiint(iv), 503 << 20), __double2loint(iv));
+            const double rr = r2 * invr, rm = rr * mi, qm = rsqrt(rm);
             const double vdotdr2 = (dx * du + dy * dv + dz * dw) * invr2;
             double dtau = 1.5 * (dts * r2 * qm) * vdotdr2;
             if (!(dtau < 1.0)) dtau = 1.0;
@@ -912,9 +916,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_steps(const int* __restr
             gmax = g1 > gmax ? g1 : gmax;
             dtau = dtp * rr * iv * vdotdr2 * (1.0 + mi * (iv * iv) * invr);
             if (!(dtau < 1.0)) dtau = 1.0;
-            // |dv|: infinite where v2 is (inf * 0 would be NaN, which no comparison keeps)
-            const double sv = __double2hiint(v2) == 0x7ff00000 ? v2 : v2 * iv;
-            const double g2 = sv * invr * idtp * (1.0 - 0.5 * dtau);
+            const double g2 = v2 * iv * invr * idtp * (1.0 - 0.5 * dtau);
             gmax = g2 > gmax ? g2 : gmax;
           } else {
             const double vdotdr2 = (dx * du + dy * dv + dz * dw) / r2;
