@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) k_p2p_plan(const int* __restrict__ tlist,
   if (ntldev) ntl = (int)*ntldev;  // device-sized launch (graph)
   const int lane = threadIdx.x & 31;
   const unsigned long long C64 = (*cost + K - 1) / K;
-  const int C = (int)(C64 < kP2PMinCost ? kP2PMinCost : C64 > 0x3fffffffull ? 0x3fffffff : C64);
+  const int C = (int)(C64 < kP2PMinCost ? kP2PMinCost : C64 > 0x7fffffffull ? 0x7fffffff : C64);
   const int nw = gridDim.x * (blockDim.x >> 5);
   for (int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < ntl; k += nw) {
     const int s = S[k];
@@ -187,13 +187,14 @@ __global__ void __launch_bounds__(256) k_p2p_plan(const int* __restrict__ tlist,
       }
       for (; m; m &= m - 1) {
         const int ts = 32 * (r0 + __ffs(m) - 1);
-        const int want = (tc_p2p_cost(s, min(32, nt - ts)) + C - 1) / C;
+        const int want = (int)(((unsigned)tc_p2p_cost(s, min(32, nt - ts)) + (unsigned)C - 1u) / (unsigned)C);
         const int B = ((s + want - 1) / want + 31) & ~31;
         const int nch = (s + B - 1) / B;
         int ib = 0;
         if (lane == 0) ib = (int)atomicAdd(&cnt[0], (unsigned)nch);
         ib = __shfl_sync(0xffffffffu, ib, 0);
-        if (ib + nch > cap) continue;  // cannot happen: the items of split rows sum to less than 2 K
+        if (ib + nch > cap) continue;  // cannot happen: a split row costs more than C, so it has less than 2 cost / C
+                                       // items, and C is at least cost / K (or as large as any row's cost)
         if (lane == 0) rows[atomicAdd(&cnt[2], 1u)] = TcP2PRow{t, ts, ib, nch};
         int p = 0;  // bodies before the window of 128 cells, four consecutive ones a lane
         for (int q0 = sb; q0 < se; q0 += 128) {
