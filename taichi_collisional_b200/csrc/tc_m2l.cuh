@@ -9,7 +9,7 @@
 // The reference's factorial table stops at (2P-1)! (kernel_fast_lean.h:127), so the scaled
 // (P, +-P) entries are zero; that is reproduced here.
 //
-// Layout: one CTA per target cell, 4 groups of 4 warps (2 at p >= 14); each group takes 32
+// Layout: a CTA takes one target cell after the other, 4 groups of 4 warps (2 at p >= 14); each group takes 32
 // (target, source) pairs at a time, one pair per lane.  Warp w of a group owns a fixed set of
 // degrees (m2l_schedule.h, balanced by a per-degree cost model) and runs every per-degree
 // step -- including the constant swap matrices, emitted as straight-line code with immediate

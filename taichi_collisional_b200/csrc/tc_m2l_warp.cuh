@@ -1,4 +1,4 @@
-// Rotation M2L in FP64, one warp per target: the form of all but the smallest systems.
+// Rotation M2L in FP64, one warp per target: the form of systems with many targets (tc_m2l_by_warp).
 //
 // The operator of tc_m2l.cuh (rotate about z, swap, rotate about x, swap, translate along z and
 // back), arranged around what bounds it on this GPU, the instruction supply.  Unrolled in registers,

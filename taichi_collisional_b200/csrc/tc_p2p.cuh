@@ -227,8 +227,11 @@ __global__ void __launch_bounds__(256) k_p2p_plan(const int* __restrict__ tlist,
 
 // ---------------------------------------------------------------------------------------
 // FP64 near field of small systems (below kP2PSmallN bodies): every leaf's source list is cut into
-// kP2PChunks pieces of as many cells, without a plan.  At 2,000 bodies a list holds at most 190
-// cells, so the pieces are even enough, and the two planning launches are saved.
+// kP2PChunks pieces of as many cells, without a plan.  The block-time-step integrator's compensation terms
+// are rounding residues of these sums, so the order of its small kicks' sums is part of what it reproduces,
+// and this is that order.  Pieces of as many cells are as even as the leaves are: near field with the pieces /
+// with work items (ms), top tree N = 1,000 and ncrit 16 0.057 / 0.069, 64 0.111 / 0.071; N = 2,000 0.064 / 0.083 and
+// 0.165 / 0.087.
 // ---------------------------------------------------------------------------------------
 constexpr int kP2PSmallN = 2048, kP2PChunks = 16;
 
@@ -640,9 +643,9 @@ __global__ void __launch_bounds__(kP2PWarps * 32) k_p2p_join(const TcP2PRow* __r
 
 // Direct summation (N below the direct threshold).  One CTA per 16 targets; its 32 half-warps take
 // every 32nd source of each 512-body tile staged in shared memory, and their sums are folded in a
-// fixed order.  A thread per target with all sources in series left 219 warps for 592 schedulers
-// at N = 7,001: 3.07 ms, now 0.15 (0.11 of FP64 pipe time).  Reads the caller's arrays and writes the
-// caller's outputs.
+// fixed order.  Bound by the FP64 pipe: 0.15 ms at N = 7,001, 0.11 of it pipe time (a thread per target with
+// all sources in series, 219 warps for 592 schedulers, takes 3.07 ms).  Reads the caller's arrays and
+// writes the caller's outputs.
 constexpr int kDirT = 16, kDirThreads = 512;
 template <bool JERK>
 __global__ void __launch_bounds__(kDirThreads) k_direct(int n, const double* __restrict__ x,
@@ -999,9 +1002,9 @@ namespace tc {
 // ---------------------------------------------------------------------------------------
 // k_p2p_mixed: the mixed-precision near field.
 //
-// One warp per target leaf, one target per lane; a last pass of r <= 16 targets runs
-// floor(32 / r) lane groups, each over every ng-th source pair of each tile (so small leaves
-// still fill the warp).  A tile takes the next 32 bodies of the target's source cells read as
+// One warp per work item (a row of up to 32 targets and all or a chunk of its sources), one target per
+// lane; a row of r <= 16 targets runs floor(32 / r) lane groups, each over every ng-th source pair of
+// each tile (so small leaves still fill the warp).  A tile takes the next 32 bodies of the target's source cells read as
 // one sequence, so small source leaves still fill it.
 //
 // Arithmetic.  Sources are staged per 32-source tile as FP32 (hi, lo) pairs of positions and of

@@ -48,7 +48,7 @@ __global__ void k_bounds_partial(int n, const double* __restrict__ x, const doub
   }
 }
 
-// one block: the partial boxes folded, then the root cell (a single thread over 592 partials took 185 us)
+// one block: the partial boxes folded side by side, then the root cell (latency: one thread needs 185 us for 592)
 constexpr int kBoundsThreads = 256;
 __global__ void __launch_bounds__(kBoundsThreads) k_bounds_final(int nblk, const double* __restrict__ part,
                                                                  TcRootInfo* root, int use_shift, double u0,
@@ -434,8 +434,15 @@ __global__ void k_tree_emit(int l, TcCells c, const TcLevels* lv, const int* __r
 }
 
 // ---------------------------------------------------------------------------------------
-// Small systems: the key sort and the levels as one CTA each.  At N = 2,000 the 32 sort launches and the
-// 66 level launches took 0.23 and 0.37 ms, nearly all of it launch and load latency.
+// Small systems: the key sort and the levels as one CTA each, bound by the latency of that CTA's loads; the
+// forms of many launches (32 for the sort, 66 for the levels) by theirs, about 0.6 ms whatever N is.
+// Tree phase, one CTA / many launches (ms):
+//   ncrit     N = 300      2,000        8,192        16,384       20,000       32,768       65,536
+//   64        0.09 / 0.46  0.12 / 0.52  0.19 / 0.60  0.29 / 0.62  0.33 / 0.63  0.49 / 0.64  0.89 / 0.67
+//   16        0.09 / 0.47  0.14 / 0.53  0.24 / 0.62  0.42 / 0.64  0.48 / 0.65  0.76 / 0.66  1.43 / 0.70
+//   4         0.11 / 0.48  0.17 / 0.53  0.36 / 0.62  0.67 / 0.65
+//   1         0.11 / 0.48  0.21 / 0.54  0.57 / 0.65  1.08 / 0.68
+// The limit is where leaves of 4 bodies gain nothing any more; wide leaves would gain up to some 25,000 bodies.
 // ---------------------------------------------------------------------------------------
 constexpr int kTreeSmallN = 16384, kTreeSmallThreads = 1024;
 

@@ -459,7 +459,11 @@ __device__ void tc_m2m_warp(int ci, const TcCells& c, cd* G, cd* SM, cd* SMd) {
 // The same sums, a warp per child: at the levels of few cells the latency of one warp that takes the
 // children in turn is the launch's time (N = 2,000, p = 8: 130 us a level with the ball search, 7 levels).
 // The children's contributions meet in shared memory and are added in child order, as tc_m2m_warp does.
-constexpr int kFewCells = 148 * 4;  // levels of at most this many inner candidates get a CTA per cell
+//
+// Levels of at most kFewCells candidates (leaves among them) get a CTA per cell.  Upward pass in ms with the
+// limit at 148 / 592 / 2,368 (p = 8, ncrit 64): N = 4,096 0.38 / 0.38 / 0.38, 20,000 0.81 / 0.50 / 0.49, 65,536
+// 1.03 / 0.91 / 0.59, 131,072 1.32 / 1.18 / 0.96, 2M 5.87 / 5.68 / 5.51: 592 is on the safe side.
+constexpr int kFewCells = 148 * 4;
 template <int P, bool JERK>
 struct TcM2MFew {
   static constexpr int NT = (P + 1) * (P + 1), NOUT = (P + 1) * (P + 2) / 2;
